@@ -57,13 +57,7 @@ WORKLOAD_TEXT = {
 # captures of a kernel on a workload at full size, keyed by (workload, kernel);
 # each entry names the capture.  A kernel without a capture reports null.
 NCU_TRAFFIC = {
-    ("c2", "k_fft_cols_pair<double,12>"): (2_312_723_797, "profiles/traffic_c2.md (mean of 3 "
-                                           "launches, one-pass dram__bytes_read/write capture)"),
-    ("c2", "k_fft_cols_tm<double,12>"): (2_383_968_341, "profiles/traffic_c2.md (mean of 3 "
-                                         "launches, one-pass dram__bytes_read/write capture)"),
     ("c2", "k_bin_scatter<32,1>"): (10_851_913_216, "profiles/traffic_c2.md"),
-    ("c2", "k_grid_tiles<double,8>"): (459_853_312, "profiles/traffic_c2.md"),
-    ("c2", "k_fft_rows<double,12>"): (2_083_898_112, "profiles/traffic_c2.md"),
 }
 
 
@@ -73,9 +67,7 @@ def plan_kernel_name(stage, nx, ny):
     lx = max(int(nx).bit_length() - 1, 0)
     return {"bin_count": "k_bin_count", "bin_scatter": "k_bin_scatter<32,1>",
             "cube_zero": "k_zero_split_tiles<double>", "grid": "k_grid_tiles<double,8>",
-            "fft": f"k_fft_rows<double,{lx}>",
-            "phase": (f"k_fft_cols_pair<double,{ly}>" if 10 <= ly <= 12
-                      else f"k_fft_cols_tm<double,{ly}>")}.get(stage, stage)
+            "fft": f"k_fft_rows<double,{lx}>", "phase": f"k_fft_cols<double,{ly}>"}.get(stage, stage)
 
 
 def fp64_gemm_tflops(dev) -> float:

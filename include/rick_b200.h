@@ -282,10 +282,10 @@ typedef struct rick_job_desc {
   double *image_real, *image_imag;       /* device [grid_size_y * grid_size_x] */
 } rick_job_desc;
 
-/* Schedule knobs of a batch: gridder records per work item, gridder blocks per
- * SM, and the column pass's form: planes_in_flight 0 keeps each pixel's running
- * sum and w-step in tensor memory (one plane per iteration); 1 or 2 keep them
- * in registers with that many planes per iteration (2: mixed form only). */
+/* Schedule knobs of a batch: gridder records per work item and gridder blocks
+ * per SM.  planes_in_flight (0, 1 or 2) is kept as given and selects nothing: the
+ * column pass has one form, each pixel's running sum and w-step in tensor memory
+ * (one plane per iteration). */
 typedef struct rick_batch_tuning {
   uint32_t max_chunk;
   int grid_blocks_per_sm;
@@ -294,7 +294,7 @@ typedef struct rick_batch_tuning {
 
 typedef struct rick_batch rick_batch;
 
-/* HBM the batch holds (cubes, column-blocked planes, records, tables). */
+/* HBM the batch holds (cubes, row-transformed planes, records, tables). */
 int rick_batch_footprint(const rick_job_desc *jobs, int njobs, int precision, uint64_t *bytes);
 /* Creates the batch on `device` (precision RICK_PREC_*).  tuning == NULL runs
  * the autotuner (times candidate schedules on the batch itself, synchronises,

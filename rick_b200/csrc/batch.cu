@@ -9,8 +9,7 @@
 // tile) bins and their work items, touched rows, column groups -- so that one
 // persistent kernel per stage serves every job; the FFT stages launch once per
 // FFT length present.  A project-written autotuner picks the gridder's work-item
-// size (records per item), its blocks per SM and the planes in flight of the
-// column pass by timing the batch itself.
+// size (records per item) and its blocks per SM by timing the batch itself.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -54,7 +53,7 @@ struct Layout {
   std::vector<int> tw_log;                          // FFT lengths with twiddles
   std::map<int, uint64_t> tw;                       // log -> offset
   uint64_t jobs = 0, row_units = 0, bin_base = 0, mask_base = 0, fft_tabs = 0, sc_tabs = 0;
-  uint64_t rowmask = 0, tilemask = 0, rowlist = 0, counts = 0;
+  uint64_t rowmask = 0, rowbits = 0, tilemask = 0, rowlist = 0, counts = 0;
   uint64_t bin_count = 0, bin_cursor = 0, item_off = 0, scan_tmp = 0, counters = 0, records = 0;
   uint64_t total = 0;
   // sizes
@@ -120,7 +119,7 @@ int plan_layout(const std::vector<rick_job_desc> &jobs, int precision, Layout &L
     return set_error(RICK_ERR_INVALID_ARG, "batch has too many rows (records are 32-bit indexed)");
   L.total_bins = (uint32_t)bins;
   L.max_records = 4 * L.total_rows;
-  for (auto &kv : L.tw) kv.second = take((uint64_t)(1 << kv.first) * 2 * vb);
+  for (auto &kv : L.tw) kv.second = take(twiddle_bytes(1 << kv.first, precision));
   L.jobs = take(sizeof(BatchJob) * n);
   L.row_units = take(8ull * (n + 1));
   L.bin_base = take(4ull * (n + 1));
@@ -128,6 +127,7 @@ int plan_layout(const std::vector<rick_job_desc> &jobs, int precision, Layout &L
   L.fft_tabs = take(4ull * (3 * n + 2));  // fft_units [n+1], col_jobs [n], col_units [n+1]
   L.sc_tabs = take(8ull * (n + 1) + 4ull * n);  // sc_units [n+1] (u64), sc_jobs [n] (u32)
   L.rowmask = take(4 * L.total_mask_words);
+  L.rowbits = take(4 * L.total_mask_words);
   L.tilemask = take(4 * L.total_tile_words);
   L.rowlist = take(4 * L.total_list);
   L.counts = take(4ull * L.total_count_words);
@@ -183,13 +183,12 @@ namespace {
 // The launch sequence of one batch run (stream-ordered; captured in the graph).
 int batch_launch(rick_batch *b, cudaStream_t st) {
   b->bl.grid_blocks_per_sm = b->tune.grid_blocks_per_sm;
-  b->fj.cols_pp = b->tune.planes_in_flight;
   RICK_CUDA(cudaMemsetAsync(b->s.counters, 0, kNumCounters * sizeof(uint64_t), st));
   RICK_CUDA(cudaMemsetAsync(b->bl.rowmask, 0, 4 * b->L.total_mask_words, st));
   RICK_CUDA(cudaMemsetAsync(b->bl.tilemask, 0, 4 * b->L.total_tile_words, st));
   RICK_TRY(bin_rows_batch(b->bl, b->s, b->tune.max_chunk, st));
   RICK_TRY(grid_tiles_batch(b->bl, b->precision, b->s, b->tune.max_chunk, st));
-  RICK_TRY(sparse_fft_lists(b->fj, st));
+  RICK_TRY(sparse_fft_lists(b->fj, b->precision, st));
   RICK_TRY(sparse_fft_rows(b->fj, b->precision, st));
   if (b->cols_gate) RICK_CUDA(cudaStreamWaitEvent(st, b->cols_gate, 0));
   RICK_TRY(sparse_fft_cols(b->fj, b->precision, st));
@@ -203,17 +202,13 @@ int build_tables(rick_batch *b, cudaStream_t st) {
   const int n = (int)b->jobs.size();
   const Layout &L = b->L;
   char *A = b->arena;
-  const bool f64 = b->precision == RICK_PREC_FP64;
   // twiddles per FFT length
   std::map<int, const void *> tw;
   for (auto &kv : L.tw) {
     const int len = 1 << kv.first;
-    std::vector<double2> t64(len);
-    std::vector<float2> t32(len);
-    make_twiddles(len, t64.data(), t32.data());
-    const void *src = f64 ? (const void *)t64.data() : (const void *)t32.data();
-    RICK_CUDA(cudaMemcpyAsync(A + kv.second, src, (size_t)len * (f64 ? 16 : 8),
-                              cudaMemcpyHostToDevice, st));
+    std::vector<char> tab(twiddle_bytes(len, b->precision));
+    make_twiddles(len, b->precision, tab.data());
+    RICK_CUDA(cudaMemcpyAsync(A + kv.second, tab.data(), tab.size(), cudaMemcpyHostToDevice, st));
     tw[kv.first] = A + kv.second;
   }
   std::vector<BatchJob> hj(n);
@@ -296,7 +291,7 @@ int build_tables(rick_batch *b, cudaStream_t st) {
   mask_base[n] = mb;
   std::vector<uint32_t> tabs(3 * n + 2, 0);
   FftJobs &f = b->fj;
-  fft_classes(hj.data(), n, f, tabs.data() + (n + 1), tabs.data() + (2 * n + 1));
+  fft_classes(hj.data(), n, b->precision, f, tabs.data() + (n + 1), tabs.data() + (2 * n + 1));
   RICK_CUDA(cudaMemcpyAsync(A + L.jobs, hj.data(), sizeof(BatchJob) * n, cudaMemcpyHostToDevice, st));
   RICK_CUDA(cudaMemcpyAsync(A + L.row_units, row_units.data(), 8 * (n + 1), cudaMemcpyHostToDevice,
                             st));
@@ -361,6 +356,7 @@ int build_tables(rick_batch *b, cudaStream_t st) {
   f.total_count_words = L.total_count_words;
   f.rowmask = bl.rowmask;
   f.tilemask = bl.tilemask;
+  f.rowbits = (uint16_t *)(A + L.rowbits);
   f.rowlist = (uint32_t *)(A + L.rowlist);
   f.counts = (uint32_t *)(A + L.counts);
 
@@ -394,9 +390,8 @@ int time_runs(rick_batch *b, int reps, float *ms) {
   return st;
 }
 
-// Coordinate descent over the gridder's records per work item, its blocks per
-// SM and the column pass's form (state in tensor memory, or planes in flight),
-// timing the batch.
+// Coordinate descent over the gridder's records per work item and its blocks
+// per SM, timing the batch.
 int autotune(rick_batch *b) {
   TuneKey key;
   key.precision = b->precision;
@@ -435,14 +430,6 @@ int autotune(rick_batch *b) {
   for (int bps : {4, 8}) {
     rick_batch_tuning t = best;
     t.grid_blocks_per_sm = bps;
-    RICK_TRY(trial(t));
-  }
-  // the column pass: state in tensor memory (0), or in registers with one or
-  // (mixed form) two planes per iteration
-  for (int pif : {1, 2}) {
-    if (pif == 2 && b->precision != RICK_PREC_MIXED) continue;
-    rick_batch_tuning t = best;
-    t.planes_in_flight = pif;
     RICK_TRY(trial(t));
   }
   b->tune = best;

@@ -318,9 +318,8 @@ BatchJob plan_job(const rick_plan *p) {
   j.cube = p->cube;
   j.blocked = p->f.blocked;
   j.table = p->s.table;
-  const bool f64 = p->d.precision == RICK_PREC_FP64;
-  j.tw_x = f64 ? (const void *)p->f.tw_x64 : (const void *)p->f.tw_x32;
-  j.tw_y = f64 ? (const void *)p->f.tw_y64 : (const void *)p->f.tw_y32;
+  j.tw_x = p->f.tw_x;
+  j.tw_y = p->f.tw_y;
   j.ltab = p->d_lm;
   j.mtab = p->d_lm + p->d.grid_size_x;
   return j;
@@ -407,7 +406,7 @@ int image_sparse_after_grid(rick_plan *p, uint64_t nrows, double resolution, dou
   // from pageable memory: the call returns once `j` has been staged
   RICK_CUDA(cudaMemcpyAsync(p->d_job, &j, sizeof(j), cudaMemcpyHostToDevice, st));
   p->fj.one = &j;
-  RICK_TRY(sparse_fft_lists(p->fj, st));
+  RICK_TRY(sparse_fft_lists(p->fj, p->d.precision, st));
   RICK_TRY(sparse_fft_rows(p->fj, p->d.precision, st));
   RICK_TRY(mark(p, p->ev[5], st));
   RICK_TRY(ensure_lm(p, nx, ny, nx, ny, resolution, st));
@@ -486,7 +485,7 @@ int rick_plan_footprint(const rick_plan_desc *desc, uint64_t *bytes) {
   const uint64_t vb = desc->precision == RICK_PREC_FP64 ? 8 : 4;
   uint64_t b = 2 * nw * nx * ny * vb;                      // cube
   if (sparse_fft_supported((int)nx, (int)ny))
-    b *= 2;                                                // + column-blocked planes
+    b *= 2;                                                // + row-transformed planes
   else
     b += std::max<uint64_t>(b / 4, 512ull << 20);          // cuFFT work (upper bound)
   b += 4 * (nbins + 1) * 4 + 4 * scan_tmp_words(nbins + 1);  // bins, items, cursor, scan
@@ -546,31 +545,28 @@ int rick_plan_create(rick_plan **out, const rick_plan_desc *desc) {
   if (st == RICK_OK && p->sparse) {
     const int nx = desc->grid_size_x, ny = desc->grid_size_y;
     A((void **)&p->f.rowmask, (size_t)nwl * p->g.nty * 4);
+    A((void **)&p->f.rowbits, (size_t)nwl * p->g.nty * 4);
     A((void **)&p->f.rowlist, (size_t)nwl * ny * 4);
     A((void **)&p->f.counts, (size_t)(1 + nwl) * 4);
     A((void **)&p->f.tilemask, (size_t)nwl * p->g.nty * ((p->g.ntx + 31) / 32) * 4);
-    A((void **)&p->f.tw_x64, (size_t)nx * sizeof(double2));
-    A((void **)&p->f.tw_y64, (size_t)ny * sizeof(double2));
-    A((void **)&p->f.tw_x32, (size_t)nx * sizeof(float2));
-    A((void **)&p->f.tw_y32, (size_t)ny * sizeof(float2));
+    A(&p->f.tw_x, twiddle_bytes(nx, desc->precision));
+    A(&p->f.tw_y, twiddle_bytes(ny, desc->precision));
     A(&p->f.blocked, p->cube_vals * p->val_bytes);
     if (st == RICK_OK) {
-      const int nmax = std::max(nx, ny);
-      double2 *t64 = (double2 *)malloc(sizeof(double2) * nmax);
-      float2 *t32 = (float2 *)malloc(sizeof(float2) * nmax);
-      if (!t64 || !t32) st = set_error(RICK_ERR_NOT_ENOUGH_MEM, "host twiddle tables");
       for (int axis = 0; axis < 2 && st == RICK_OK; axis++) {
         const int n = axis == 0 ? nx : ny;
-        make_twiddles(n, t64, t32);
-        cudaError_t e = cudaMemcpy(axis == 0 ? p->f.tw_x64 : p->f.tw_y64, t64, sizeof(double2) * n,
-                                   cudaMemcpyHostToDevice);
-        if (e == cudaSuccess)
-          e = cudaMemcpy(axis == 0 ? p->f.tw_x32 : p->f.tw_y32, t32, sizeof(float2) * n,
-                         cudaMemcpyHostToDevice);
+        const size_t bytes = twiddle_bytes(n, desc->precision);
+        void *tab = malloc(bytes);
+        if (!tab) {
+          st = set_error(RICK_ERR_NOT_ENOUGH_MEM, "host twiddle table");
+          break;
+        }
+        make_twiddles(n, desc->precision, tab);
+        const cudaError_t e =
+            cudaMemcpy(axis == 0 ? p->f.tw_x : p->f.tw_y, tab, bytes, cudaMemcpyHostToDevice);
         if (e != cudaSuccess) st = cuda_status(e, "cudaMemcpy(twiddles)", __FILE__, __LINE__);
+        free(tab);
       }
-      free(t64);
-      free(t32);
     }
     A((void **)&p->d_job, sizeof(BatchJob));
     A((void **)&p->d_fft_tabs, 8 * sizeof(uint32_t));
@@ -579,7 +575,7 @@ int rick_plan_create(rick_plan **out, const rick_plan_desc *desc) {
       FftJobs &fj = p->fj;
       BatchJob hj = plan_job(p);
       uint32_t tabs[8] = {};
-      fft_classes(&hj, 1, fj, tabs + 2, tabs + 3);
+      fft_classes(&hj, 1, desc->precision, fj, tabs + 2, tabs + 3);
       const uint64_t mb[2] = {0, (uint64_t)nwl * p->g.nty};
       fj.jobs = p->d_job;
       fj.njobs = 1;
@@ -589,8 +585,10 @@ int rick_plan_create(rick_plan **out, const rick_plan_desc *desc) {
       fj.mask_base = p->d_mask_base;
       fj.total_mask_words = mb[1];
       fj.total_count_words = 1 + nwl;
+      fj.cols_parts = column_parts(desc->precision, nx, ny, nwl);
       fj.rowmask = p->f.rowmask;
       fj.tilemask = p->f.tilemask;
+      fj.rowbits = p->f.rowbits;
       fj.rowlist = p->f.rowlist;
       fj.counts = p->f.counts;
       cudaError_t e = cudaMemcpy(p->d_fft_tabs, tabs, sizeof(tabs), cudaMemcpyHostToDevice);
@@ -620,8 +618,8 @@ int rick_plan_destroy(rick_plan *p) {
     if (e) cudaEventDestroy(e);
   void *ptrs[] = {p->cube, p->s.bin_count, p->s.bin_cursor, p->s.item_off, p->s.scan_tmp,
                   p->s.counters, p->s.records, p->s.table, p->d_lm, p->fft_work, p->h_rows_d,
-                  p->d_img, p->d_stage, p->d_norm, p->f.rowmask, p->f.rowlist, p->f.counts,
-                  p->f.tw_x64, p->f.tw_y64, p->f.tw_x32, p->f.tw_y32, p->f.blocked,
+                  p->d_img, p->d_stage, p->d_norm, p->f.rowmask, p->f.rowbits, p->f.rowlist, p->f.counts,
+                  p->f.tw_x, p->f.tw_y, p->f.blocked,
                   p->f.tilemask, p->d_job, p->d_fft_tabs, p->d_mask_base};
   for (void *q : ptrs)
     if (q) cudaFree(q);

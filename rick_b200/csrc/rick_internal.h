@@ -85,12 +85,12 @@ struct Scratch {
 // Scratch of the sparse-aware FFT (fft.cu).
 struct FftScratch {
   uint32_t *rowmask = nullptr;  // [nw * nty] bit k%32 of word (w, k/32): row k touched
+  uint16_t *rowbits = nullptr;  // [nw * ny / 16] the row mask by column-pass thread
   uint32_t *rowlist = nullptr;  // [nw * ny] touched (plane, row) ids
   uint32_t *counts = nullptr;   // [1 + nw] touched rows, then touched rows per plane
   uint32_t *tilemask = nullptr; // [nw * nty * ceil(ntx/32)] bit tx: tile (w, ty, tx) holds records
-  double2 *tw_x64 = nullptr, *tw_y64 = nullptr;  // per-pass twiddles of the two axes
-  float2 *tw_x32 = nullptr, *tw_y32 = nullptr;
-  void *blocked = nullptr;      // row-transformed planes, column-blocked (cube-sized)
+  void *tw_x = nullptr, *tw_y = nullptr;  // twiddles of the two axes
+  void *blocked = nullptr;      // row-transformed planes by column units (cube-sized)
 };
 
 // One job of a batch (batch.cu), as the batch kernels see it: the job's
@@ -113,9 +113,9 @@ struct BatchJob {
   const double *uu, *vv, *ww;      // rows (device)
   const float *weight, *vis_re, *vis_im;
   void *cube;                      // [nw][ny][nx] complex (T)
-  void *blocked;                   // column-blocked row transforms (cube-sized)
+  void *blocked;                   // row transforms by column units (cube-sized)
   const double *table;             // 1-D kernel table (5*support)
-  const void *tw_x, *tw_y;         // per-pass twiddles of the two axes (T)
+  const void *tw_x, *tw_y;         // twiddles of the two axes
   const double *ltab, *mtab;       // phase tables (nx, ny)
   double wmin, dw_phase, dwnorm, norm;
   int phase_on;
@@ -147,19 +147,20 @@ struct FftJobs {
   uint64_t total_mask_words = 0;
   uint32_t total_count_words = 0;
   uint32_t *rowmask = nullptr, *tilemask = nullptr, *rowlist = nullptr, *counts = nullptr;
+  uint16_t *rowbits = nullptr;          // two entries per row-mask word
+  int cols_parts = 1;                   // blocks a unit's planes are dealt to (one job)
   int n_row_cls = 0, n_col_cls = 0;
   FftClass row_cls[8], col_cls[8];
-  int cols_pp = 2;                   // planes per column-pass iteration allowed (1 or 2)
   // a set of one job (a plan): its host copy; the FFT kernels then take the
   // job as kernel parameters instead of reading the device table
   const BatchJob *one = nullptr;
 };
 
-// Rows (columns) one block of the row (column) pass transforms at length 2^logn:
-// a row takes 2^logn / 8 threads, a block max(256, 2^logn / 8).
-__host__ __device__ inline int fft_rows_per_block(int logn) {
-  const int g = (1 << logn) / 8;
-  return (g > 256 ? g : 256) / g;
+// Transforms (of 2^logn points, 16 values a thread) that a block of the FFT passes
+// runs at once (fft_core.cuh, Shape::kGroups).
+__host__ __device__ inline int fft_groups_per_block(int logn) {
+  const int g = (1 << logn) / 16;
+  return g >= 128 ? 1 : 128 / g;
 }
 
 enum Counter : int {
@@ -194,7 +195,8 @@ int grid_tiles(const Geometry &g, int kernel, int precision, Scratch &s, void *c
 int zero_split_tiles(const Geometry &g, int precision, Scratch &s, void *cube, cudaStream_t st);
 // Sparse-aware FFT (fft.cu).
 bool sparse_fft_supported(int nx, int ny);
-void make_twiddles(int n, double2 *t64, float2 *t32);
+size_t twiddle_bytes(int n, int precision);
+void make_twiddles(int n, int precision, void *tab);  // twiddle_bytes of host memory
 void phase_tables(int xaxis, int yaxis, int xaxistot, int yaxistot, double resolution,
                   double *l, double *m);
 // Planes w_first .. w_first+nw-1 of an nw_total-plane cube (phase_correction
@@ -257,9 +259,11 @@ int grid_tiles_batch(const BatchLaunch &b, int precision, Scratch &s, uint32_t m
 // The sparse-aware FFT stages (fft.cu) of a set of jobs.  fft_classes fills the
 // classes and the host copies of col_jobs / col_units (njobs and njobs + 1
 // entries) from the host copy of the jobs (sorted by logx).
-void fft_classes(const BatchJob *host_jobs, int njobs, FftJobs &f, uint32_t *col_jobs,
-                 uint32_t *col_units);
-int sparse_fft_lists(const FftJobs &f, cudaStream_t st);  // row lists and row-pass units
+void fft_classes(const BatchJob *host_jobs, int njobs, int precision, FftJobs &f,
+                 uint32_t *col_jobs, uint32_t *col_units);
+// Blocks the planes of one job's column pass are dealt to (FftJobs::cols_parts).
+int column_parts(int precision, int nx, int ny, int nw);
+int sparse_fft_lists(const FftJobs &f, int precision, cudaStream_t st);  // row lists and row-pass units
 int sparse_fft_rows(const FftJobs &f, int precision, cudaStream_t st);
 int sparse_fft_cols(const FftJobs &f, int precision, cudaStream_t st);
 

@@ -74,7 +74,7 @@ struct rick_server {
   // blocks allocate tensor memory; see rick_batch::cols_gate); batches are
   // launched by the scheduler thread alone, in order
   cudaEvent_t cols_gate = nullptr;
-  rick_batch_tuning tune{2048, 6, 1};
+  rick_batch_tuning tune{2048, 6, 0};
   rick_server_stats stats{};
 };
 
