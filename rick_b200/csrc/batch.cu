@@ -55,6 +55,7 @@ struct Layout {
   uint64_t jobs = 0, row_units = 0, bin_base = 0, mask_base = 0, fft_tabs = 0, sc_tabs = 0;
   uint64_t rowmask = 0, rowbits = 0, tilemask = 0, rowlist = 0, counts = 0;
   uint64_t bin_count = 0, bin_cursor = 0, item_off = 0, scan_tmp = 0, counters = 0, records = 0;
+  uint64_t clear = 0, clear_bytes = 0;
   uint64_t total = 0;
   // sizes
   uint64_t total_rows = 0, total_row_units = 0, max_records = 0;
@@ -126,16 +127,19 @@ int plan_layout(const std::vector<rick_job_desc> &jobs, int precision, Layout &L
   L.mask_base = take(8ull * (n + 1));
   L.fft_tabs = take(4ull * (3 * n + 2));  // fft_units [n+1], col_jobs [n], col_units [n+1]
   L.sc_tabs = take(8ull * (n + 1) + 4ull * n);  // sc_units [n+1] (u64), sc_jobs [n] (u32)
-  L.rowmask = take(4 * L.total_mask_words);
   L.rowbits = take(4 * L.total_mask_words);
-  L.tilemask = take(4 * L.total_tile_words);
   L.rowlist = take(4 * L.total_list);
+  L.item_off = take(4ull * (bins + 1));
+  L.scan_tmp = take(4ull * scan_tmp_words(bins + 1));
+  // cleared together before every run
+  L.clear = off;
+  L.counters = take(8ull * kNumCounters);
+  L.rowmask = take(4 * L.total_mask_words);
+  L.tilemask = take(4 * L.total_tile_words);
   L.counts = take(4ull * L.total_count_words);
   L.bin_count = take(4ull * (bins + 1));
   L.bin_cursor = take(4ull * (bins + 1));
-  L.item_off = take(4ull * (bins + 1));
-  L.scan_tmp = take(4ull * scan_tmp_words(bins + 1));
-  L.counters = take(8ull * kNumCounters);
+  L.clear_bytes = off - L.clear;
   L.records = take(sizeof(RecF64) * std::max<uint64_t>(L.max_records, 1));
   L.total = off;
   return RICK_OK;
@@ -183,9 +187,7 @@ namespace {
 // The launch sequence of one batch run (stream-ordered; captured in the graph).
 int batch_launch(rick_batch *b, cudaStream_t st) {
   b->bl.grid_blocks_per_sm = b->tune.grid_blocks_per_sm;
-  RICK_CUDA(cudaMemsetAsync(b->s.counters, 0, kNumCounters * sizeof(uint64_t), st));
-  RICK_CUDA(cudaMemsetAsync(b->bl.rowmask, 0, 4 * b->L.total_mask_words, st));
-  RICK_CUDA(cudaMemsetAsync(b->bl.tilemask, 0, 4 * b->L.total_tile_words, st));
+  RICK_CUDA(cudaMemsetAsync(b->arena + b->L.clear, 0, b->L.clear_bytes, st));
   RICK_TRY(bin_rows_batch(b->bl, b->s, b->tune.max_chunk, st));
   RICK_TRY(grid_tiles_batch(b->bl, b->precision, b->s, b->tune.max_chunk, st));
   RICK_TRY(sparse_fft_lists(b->fj, b->precision, st));
@@ -228,8 +230,7 @@ int build_tables(rick_batch *b, cudaStream_t st) {
     g.half = (d.w_support - 1) / 2;
     g.ntx = (g.nx + kTile - 1) / kTile;
     g.nty = (g.ny + kTile - 1) / kTile;
-    g.dx = 1.0 / g.nx;  // init.c:11-12
-    g.dw = 1.0 / g.nw;
+    g.set_spacing(1.0 / g.nx, 1.0 / g.nw);  // init.c:11-12
     g.w_supporth = (double)g.half * (1.0 / (double)g.nx);  // init.c:13
     g.select_sector0 = d.row_selection == RICK_ROWS_SECTOR0;
     J.kernel = d.kernel;
@@ -239,11 +240,9 @@ int build_tables(rick_batch *b, cudaStream_t st) {
     J.nchan = d.freq_per_chan;
     J.npol = d.polarizations;
     {
-      const uint32_t nv = d.freq_per_chan * d.polarizations;
-      const bool aligned = ((uintptr_t)d.vis_real % 16 == 0) && ((uintptr_t)d.vis_img % 16 == 0);
-      J.scatter_v4 = aligned && nv % 4 == 0 &&
-                     (d.polarizations == 1 || d.polarizations == 2 || d.polarizations == 4);
-      J.scatter_lanes = lanes_per_row(J.scatter_v4 ? nv / 4 : nv);
+      const uint64_t nv = (uint64_t)d.freq_per_chan * d.polarizations;
+      J.scatter_vec = sample_vector(d.vis_real, d.vis_img, nv, d.polarizations);
+      J.scatter_lanes = lanes_per_row(nv / J.scatter_vec);
     }
     J.bin_base = bb;
     J.counts_base = cb;
@@ -299,7 +298,7 @@ int build_tables(rick_batch *b, cudaStream_t st) {
   RICK_CUDA(cudaMemcpyAsync(A + L.mask_base, mask_base.data(), 8 * (n + 1), cudaMemcpyHostToDevice,
                             st));
   RICK_CUDA(cudaMemcpyAsync(A + L.fft_tabs, tabs.data(), 4 * tabs.size(), cudaMemcpyHostToDevice, st));
-  // sample-pass schedules: the jobs grouped by (lanes per row, 16-byte loads)
+  // sample-pass schedules: the jobs grouped by (lanes per row, samples per load)
   BatchLaunch &bl = b->bl;
   {
     std::vector<uint64_t> sc_units(n + 1, 0);
@@ -307,12 +306,12 @@ int build_tables(rick_batch *b, cudaStream_t st) {
     int k = 0;
     uint64_t acc = 0;
     bl.n_sc = 0;
-    for (int v4 = 1; v4 >= 0; v4--)
+    for (int vec = 4; vec >= 1; vec /= 2)
       for (int lanes = 1; lanes <= 32; lanes *= 2) {
         const int lo = k;
         uint64_t units = 0;
         for (int j = 0; j < n; j++) {
-          if (hj[j].scatter_v4 != v4 || hj[j].scatter_lanes != lanes) continue;
+          if (hj[j].scatter_vec != vec || hj[j].scatter_lanes != lanes) continue;
           sc_jobs[k] = (uint32_t)j;
           sc_units[k] = acc;
           const uint64_t u = (hj[j].nrows + 31) / 32;
@@ -320,7 +319,7 @@ int build_tables(rick_batch *b, cudaStream_t st) {
           units += u;
           k++;
         }
-        if (k > lo && units > 0) bl.sc[bl.n_sc++] = ScatterClass{lanes, v4 != 0, lo, k, units};
+        if (k > lo && units > 0) bl.sc[bl.n_sc++] = ScatterClass{lanes, vec, lo, k, units};
       }
     sc_units[n] = acc;
     RICK_CUDA(cudaMemcpyAsync(A + L.sc_tabs, sc_units.data(), 8 * (n + 1), cudaMemcpyHostToDevice,
@@ -353,7 +352,6 @@ int build_tables(rick_batch *b, cudaStream_t st) {
   f.col_units = f.fft_units + (2 * n + 1);
   f.mask_base = (const uint64_t *)(A + L.mask_base);
   f.total_mask_words = L.total_mask_words;
-  f.total_count_words = L.total_count_words;
   f.rowmask = bl.rowmask;
   f.tilemask = bl.tilemask;
   f.rowbits = (uint16_t *)(A + L.rowbits);

@@ -12,8 +12,9 @@
 // sort by (plane, tile), so the gridder reads only the rows of the tile it owns.
 //
 // Cell assignment is bit-exact with w-stacking.cu:143-149: FP64 IEEE division
-// by dx / dw and truncation toward zero, written with explicit round-to-nearest
-// intrinsics so that no multiply-add contraction can change a rounding.
+// by dx / dw (or, for a power of two, the product with its inverse: the same bits)
+// and truncation toward zero, written with explicit round-to-nearest intrinsics so
+// that no multiply-add contraction can change a rounding.
 #include <algorithm>
 
 #include "rick_internal.h"
@@ -50,9 +51,14 @@ __device__ __forceinline__ bool in_sector0(double v, const Geometry &g) {
 // rows of the other shards' planes are skipped (counted apart).
 __device__ __forceinline__ RowPos row_position(double u, double v, double w, const Geometry &g) {
   RowPos p;
-  p.pu = __ddiv_rn(u, g.dx);
-  p.pv = __ddiv_rn(v, g.dx);
-  const double wi = __ddiv_rn(w, g.dw);
+  if (g.inv_dx > 0.0) {
+    p.pu = __dmul_rn(u, g.inv_dx);
+    p.pv = __dmul_rn(v, g.inv_dx);
+  } else {
+    p.pu = __ddiv_rn(u, g.dx);
+    p.pv = __ddiv_rn(v, g.dx);
+  }
+  const double wi = g.inv_dw > 0.0 ? __dmul_rn(w, g.inv_dw) : __ddiv_rn(w, g.dw);
   p.gw = (int)wi;
   p.gu = (int)p.pu;
   p.gv = (int)p.pv;
@@ -65,9 +71,30 @@ __device__ __forceinline__ RowPos row_position(double u, double v, double w, con
   return p;
 }
 
-// Bins of the (up to 2x2) tiles a footprint touches, kNoBin for unused slots.
+// Bins of the (up to 2x2) tiles a footprint touches, kNoBin for unused slots
+// (slot 0 is used if any is).
 __device__ __forceinline__ void footprint_bins(const RowPos &p, const Geometry &g,
                                                uint32_t bins[4]) {
+  bins[0] = bins[1] = bins[2] = bins[3] = kNoBin;
+  if (!p.keep) return;
+  const int jmin = max(p.gu - g.half, 0), jmax = min(p.gu + g.half, g.nx - 1);
+  const int kmin = max(p.gv - g.half, 0), kmax = min(p.gv + g.half, g.ny - 1);
+  if (jmin > jmax || kmin > kmax) return;  // footprint entirely off the grid
+  const uint32_t tx0 = (uint32_t)jmin / kTile, ty0 = (uint32_t)kmin / kTile;
+  const bool right = (uint32_t)jmax / kTile > tx0, down = (uint32_t)kmax / kTile > ty0;
+  const uint32_t b = ((uint32_t)p.gw * g.nty + ty0) * g.ntx + tx0;  // bins fit 32 bits
+  bins[0] = b;
+  if (right) bins[1] = b + 1;
+  if (down) bins[2] = b + g.ntx;
+  if (right && down) bins[3] = b + g.ntx + 1;
+}
+
+// The same bins, packed to the front by a loop over the tiles, for the streaming
+// sample pass: with the straight-line form the compiler keeps fewer of that pass's
+// sample loads in flight (48 registers for 62: 2.94 ms for 1.75 at 5.1M rows of 256
+// samples).
+__device__ __forceinline__ void footprint_bins_packed(const RowPos &p, const Geometry &g,
+                                                      uint32_t bins[4]) {
   bins[0] = bins[1] = bins[2] = bins[3] = kNoBin;
   if (!p.keep) return;
   const int jmin = max(p.gu - g.half, 0), jmax = min(p.gu + g.half, g.nx - 1);
@@ -106,12 +133,15 @@ __device__ __forceinline__ void cache_init(CountCache *c) {
   }
   __syncthreads();
 }
-__device__ __forceinline__ void cache_add(CountCache *c, uint32_t bin, uint32_t n,
+__device__ __forceinline__ void cache_add(CountCache *c, uint32_t bin,
                                           uint32_t *__restrict__ bin_count) {
   const uint32_t h = (bin * 2654435761u) >> (32 - 11);  // multiplicative hash, 11 bits
-  const uint32_t k = atomicCAS(&c->key[h], kNoBin, bin);
-  if (k == kNoBin || k == bin) atomicAdd(&c->cnt[h], n);
-  else atomicAdd(&bin_count[bin], n);
+  // a taken slot is read, not compare-and-swapped: the lanes of a warp that share a
+  // bin would take turns at the swap, while the hardware adds their ones together
+  uint32_t k = *(volatile uint32_t *)&c->key[h];
+  if (k == kNoBin) k = atomicCAS(&c->key[h], kNoBin, bin);
+  if (k == kNoBin || k == bin) atomicAdd(&c->cnt[h], 1u);
+  else atomicAdd(&bin_count[bin], 1u);
 }
 __device__ __forceinline__ void cache_flush(CountCache *c, uint32_t *__restrict__ bin_count) {
   __syncthreads();
@@ -119,34 +149,63 @@ __device__ __forceinline__ void cache_flush(CountCache *c, uint32_t *__restrict_
     if (c->cnt[i]) atomicAdd(&bin_count[c->key[i]], c->cnt[i]);
 }
 
-// Pass 1 over rows base..base+31 (one per lane): histogram of records per bin.
-// Every lane adds its row's bins into the block's cache (the uv centre is
-// dense: hot bins are counted in shared memory, not by global atomics; a
-// warp-level match before the cache measured slower).  Returns 1 on a lane
-// whose row was dropped; `other` counts rows of other shards.
-__device__ __forceinline__ uint32_t count_rows(const double *__restrict__ uu,
-                                               const double *__restrict__ vv,
-                                               const double *__restrict__ ww, uint64_t nrows,
-                                               const Geometry &g, uint64_t base,
-                                               uint32_t bin_base, uint32_t *__restrict__ bin_count,
-                                               uint32_t &other, CountCache *cache) {
+// Pass 1 over 32-row units u0..u1-1 of one job (rows 32 u .., one per lane):
+// histogram of records per bin.  The coordinates of four units are read at once.
+// Every lane adds its row's bins into the block's cache (the uv centre is dense:
+// hot bins are counted in shared memory, not by global atomics; a warp-level match
+// before the cache measured slower).  Counts rows dropped and rows of other shards.
+constexpr int kCountUnits = 4;
+__device__ __forceinline__ void count_units(const double *__restrict__ uu,
+                                            const double *__restrict__ vv,
+                                            const double *__restrict__ ww, uint64_t nrows,
+                                            const Geometry &g, uint64_t u0, uint64_t u1,
+                                            uint32_t bin_base, uint32_t *__restrict__ bin_count,
+                                            uint32_t &dropped, uint32_t &other,
+                                            CountCache *cache) {
   const unsigned lane = lane_id();
-  const uint64_t i = base + lane;
-  RowPos p;
-  p.keep = false;
-  uint32_t dropped = 0;
-  if (i < nrows) {
-    p = row_position(uu[i], vv[i], ww[i], g);
-    dropped = (p.keep || p.other) ? 0u : 1u;
-    other += p.other ? 1u : 0u;
-  }
-  uint32_t bins[4];
-  footprint_bins(p, g, bins);
-  offset_bins(bins, bin_base);
+  for (uint64_t u = u0; u < u1; u += kCountUnits) {
+    double x[kCountUnits], y[kCountUnits], z[kCountUnits];
 #pragma unroll
-  for (int s = 0; s < 4; s++)
-    if (bins[s] != kNoBin) cache_add(cache, bins[s], 1u, bin_count);
-  return dropped;
+    for (int k = 0; k < kCountUnits; k++) {
+      const uint64_t i = (u + k) * 32 + lane;
+      x[k] = y[k] = z[k] = 0.0;
+      if (u + k < u1 && i < nrows) {
+        x[k] = __ldg(uu + i);
+        y[k] = __ldg(vv + i);
+        z[k] = __ldg(ww + i);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kCountUnits; k++) {
+      const uint64_t i = (u + k) * 32 + lane;
+      if (u + k >= u1 || i >= nrows) continue;
+      const RowPos p = row_position(x[k], y[k], z[k], g);
+      dropped += (p.keep || p.other) ? 0u : 1u;
+      other += p.other ? 1u : 0u;
+      uint32_t bins[4];
+      footprint_bins(p, g, bins);
+      offset_bins(bins, bin_base);
+#pragma unroll
+      for (int s = 0; s < 4; s++)
+        if (bins[s] != kNoBin) cache_add(cache, bins[s], bin_count);
+    }
+  }
+}
+
+// Contiguous run of `total` units that warp `warp` of `nwarps` takes: neighbouring
+// units share tiles (and, in a batch, the job).
+__device__ __forceinline__ void warp_run(uint64_t total, uint64_t warp, uint64_t nwarps,
+                                         uint64_t &u0, uint64_t &u1) {
+  const uint64_t per = (total + nwarps - 1) / nwarps;
+  u0 = min(total, warp * per);
+  u1 = min(total, u0 + per);
+}
+
+// A record in one 32-byte store (a sector).
+__device__ __forceinline__ void store_record(RecF64 *to, const RecF64 &r) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(to), "d"(r.sre), "d"(r.sim),
+               "d"(r.pu), "d"(r.pv)
+               : "memory");
 }
 
 __device__ __forceinline__ void add_dropped(uint32_t dropped, uint32_t other, uint64_t *counters) {
@@ -158,57 +217,127 @@ __device__ __forceinline__ void add_dropped(uint32_t dropped, uint32_t other, ui
   if (lane_id() == 0 && other) atomicAdd((unsigned long long *)&counters[kCntOtherShard], other);
 }
 
-__global__ void k_bin_count(const double *__restrict__ uu, const double *__restrict__ vv,
-                            const double *__restrict__ ww, uint64_t nrows, Geometry g,
-                            uint32_t *__restrict__ bin_count, uint64_t *__restrict__ counters) {
+__global__ void __launch_bounds__(256, 4)
+    k_bin_count(const double *__restrict__ uu, const double *__restrict__ vv,
+                const double *__restrict__ ww, uint64_t nrows, Geometry g,
+                uint32_t *__restrict__ bin_count, uint64_t *__restrict__ counters) {
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
   __shared__ CountCache cache;
   cache_init(&cache);
   uint32_t dropped = 0, other = 0;
-  for (uint64_t base = warp * 32; base < nrows; base += nwarps * 32)
-    dropped += count_rows(uu, vv, ww, nrows, g, base, 0, bin_count, other, &cache);
+  uint64_t u0, u1;
+  warp_run((nrows + 31) / 32, warp, nwarps, u0, u1);
+  count_units(uu, vv, ww, nrows, g, u0, u1, 0, bin_count, dropped, other, &cache);
   cache_flush(&cache, bin_count);
   add_dropped(dropped, other, counters);
 }
 
-// The same over every job of a batch: one warp per 32-row unit of one job.
-__global__ void k_bin_count_batch(const BatchJob *__restrict__ jobs, int njobs,
-                                  const uint64_t *__restrict__ row_units, uint64_t total_units,
-                                  uint32_t *__restrict__ bin_count,
-                                  uint64_t *__restrict__ counters) {
+// The same over every job of a batch: a warp's run of 32-row units, job by job.
+__global__ void __launch_bounds__(256, 4)
+    k_bin_count_batch(const BatchJob *__restrict__ jobs, int njobs,
+                      const uint64_t *__restrict__ row_units, uint64_t total_units,
+                      uint32_t *__restrict__ bin_count, uint64_t *__restrict__ counters) {
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
   __shared__ CountCache cache;
   cache_init(&cache);
   uint32_t dropped = 0, other = 0;
-  for (uint64_t u = warp; u < total_units; u += nwarps) {
-    const int j = batch_job_of(row_units, njobs, u);
-    const BatchJob &J = jobs[j];
-    const Geometry g = J.g;
-    dropped += count_rows(J.uu, J.vv, J.ww, J.nrows, g, (u - row_units[j]) * 32, J.bin_base,
-                          bin_count, other, &cache);
+  uint64_t u, u1;
+  warp_run(total_units, warp, nwarps, u, u1);
+  if (u < u1) {
+    int j = batch_job_of(row_units, njobs, u);
+    while (u < u1) {
+      while (row_units[j + 1] <= u) j++;
+      const uint64_t first = row_units[j], end = min(u1, row_units[j + 1]);
+      const BatchJob &J = jobs[j];
+      count_units(J.uu, J.vv, J.ww, J.nrows, J.g, u - first, end - first, J.bin_base, bin_count,
+                  dropped, other, &cache);
+      u = end;
+    }
   }
   cache_flush(&cache, bin_count);
   add_dropped(dropped, other, counters);
 }
 
-// Work items of the gridder: a bin with c records is split into ceil(c/max_chunk)
-// chunks (0 for an empty bin) so that no item is much larger than another.
-__global__ void k_item_count(const uint32_t *__restrict__ bin_off, uint64_t nbins,
-                             uint32_t max_chunk, uint32_t *__restrict__ item_count) {
-  for (uint64_t b = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; b <= nbins;
-       b += gridDim.x * (uint64_t)blockDim.x) {
-    uint32_t c = b < nbins ? bin_off[b + 1] - bin_off[b] : 0;
-    item_count[b] = (c + max_chunk - 1) / max_chunk;
+// N consecutive samples in one streaming load.
+template <int N> struct SampleVec;
+template <> struct SampleVec<4> { using t = float4; };
+template <> struct SampleVec<2> { using t = float2; };
+template <> struct SampleVec<1> { using t = float; };
+template <int N>
+__device__ __forceinline__ void load_samples(const float *__restrict__ p, float (&x)[N]) {
+  const auto v = __ldcs(reinterpret_cast<const typename SampleVec<N>::t *>(p));
+  if constexpr (N == 4) {
+    x[0] = v.x;
+    x[1] = v.y;
+    x[2] = v.z;
+    x[3] = v.w;
+  } else if constexpr (N == 2) {
+    x[0] = v.x;
+    x[1] = v.y;
+  } else {
+    x[0] = v;
   }
 }
 
-// Pass 2 over rows base..base+31: row sums and record scatter.  Each group of
-// G lanes reduces one row's samples with 16-byte loads (V4) or scalar loads;
-// after G rounds every lane holds the sum of "its" row, and the records are
-// scattered one row per lane with warp-combined cursor increments.
-template <int G, bool V4, bool SHARD>
+// One row's sums by one lane (loads of N, two loads of each array in flight): each
+// weight*vis product is the FP32 product, a sample whose real part is NaN is skipped.
+template <int N>
+__device__ __forceinline__ void row_sums(const float *__restrict__ wrow,
+                                         const float *__restrict__ re,
+                                         const float *__restrict__ im, uint32_t npol, uint32_t nv,
+                                         double &sre, double &sim) {
+  if constexpr (N > 1) {
+    // the polarisations (1, 2 or 4, sample_vector) repeat within a load: component c
+    // of every load is polarisation c mod npol
+    float wc[N];
+#pragma unroll
+    for (int c = 0; c < N; c++) wc[c] = __ldg(wrow + (c & (npol - 1)));
+    auto add = [&](const float (&ar)[N], const float (&bi)[N]) {
+#pragma unroll
+      for (int c = 0; c < N; c++) {
+        if (!isnan(ar[c])) {
+          sre += (double)__fmul_rn(wc[c], ar[c]);
+          sim += (double)__fmul_rn(wc[c], bi[c]);
+        }
+      }
+    };
+    const uint32_t nq = nv / N;
+    uint32_t q = 0;
+    float a0[N], b0[N], a1[N], b1[N];
+    for (; q + 1 < nq; q += 2) {
+      load_samples<N>(re + q * N, a0);
+      load_samples<N>(im + q * N, b0);
+      load_samples<N>(re + q * N + N, a1);
+      load_samples<N>(im + q * N + N, b1);
+      add(a0, b0);
+      add(a1, b1);
+    }
+    if (q < nq) {
+      load_samples<N>(re + q * N, a0);
+      load_samples<N>(im + q * N, b0);
+      add(a0, b0);
+    }
+  } else {
+    for (uint32_t q = 0; q < nv; q++) {
+      const float a = __ldcs(re + q);
+      if (!isnan(a)) {
+        const float wq = __ldg(wrow + (q % npol));
+        sre += (double)__fmul_rn(wq, a);
+        sim += (double)__fmul_rn(wq, __ldcs(im + q));
+      }
+    }
+  }
+}
+
+// Pass 2, streaming: rows base..base+31 of a warp.  Each group of G lanes reduces
+// one row's samples in loads of N; after G rounds every lane holds the sum of "its"
+// row, and the records are scattered one row per lane with warp-combined cursor
+// increments.  HBM-bound for long rows (5.1M rows of 256 samples: 10.8 GB in 1.75 ms,
+// 0.95 of the measured copy rate); rows of eight loads run four lanes a row (3.8M
+// rows of 32 samples: 0.29 ms, against 0.72 with a lane a row and 0.35 with eight).
+template <int G, int N, bool SHARD>
 __device__ __forceinline__ void scatter_rows(
     const double *__restrict__ uu, const double *__restrict__ vv, const double *__restrict__ ww,
     const float *__restrict__ weight, const float *__restrict__ vis_re,
@@ -231,7 +360,7 @@ __device__ __forceinline__ void scatter_rows(
     q.keep = false;
     if (i_own < nrows) q = row_position(uu[i_own], vv[i_own], ww[i_own], g);
     uint32_t qb[4];
-    footprint_bins(q, g, qb);
+    footprint_bins_packed(q, g, qb);
     need = qb[0] != kNoBin;
   }
   double my_re = 0.0, my_im = 0.0;
@@ -242,21 +371,21 @@ __device__ __forceinline__ void scatter_rows(
     const bool need_i = __shfl_sync(kFull, need, round * R + grp);
     if (i < nrows && need_i) {
       const float *wrow = weight + i * npol;
-      if (V4) {
-        // npol divides 4, so component c of every float4 is polarisation c % npol
-        float wc[4];
+      if (N > 1) {
+        // the polarisations repeat within a load (sample_vector): component c of
+        // every load is polarisation c % npol
+        float wc[N];
 #pragma unroll
-        for (int c = 0; c < 4; c++) wc[c] = __ldg(wrow + (c % npol));
-        const float4 *r4 = reinterpret_cast<const float4 *>(vis_re + i * nv);
-        const float4 *i4 = reinterpret_cast<const float4 *>(vis_im + i * nv);
-        const uint64_t nq = nv / 4;
+        for (int c = 0; c < N; c++) wc[c] = __ldg(wrow + (c % npol));
+        const float *re = vis_re + i * nv, *im = vis_im + i * nv;
+        const uint64_t nq = nv / N;
 #pragma unroll 2
         for (uint64_t q = sub; q < nq; q += G) {
-          const float4 a = __ldcs(r4 + q);
-          const float4 b = __ldcs(i4 + q);
-          const float ar[4] = {a.x, a.y, a.z, a.w}, bi[4] = {b.x, b.y, b.z, b.w};
+          float ar[N], bi[N];
+          load_samples<N>(re + q * N, ar);
+          load_samples<N>(im + q * N, bi);
 #pragma unroll
-          for (int c = 0; c < 4; c++) {
+          for (int c = 0; c < N; c++) {
             if (!isnan(ar[c])) {
               sre += (double)__fmul_rn(wc[c], ar[c]);
               sim += (double)__fmul_rn(wc[c], bi[c]);
@@ -294,7 +423,7 @@ __device__ __forceinline__ void scatter_rows(
   p.keep = false;
   if (i < nrows) p = row_position(uu[i], vv[i], ww[i], g);
   uint32_t bins[4];
-  footprint_bins(p, g, bins);
+  footprint_bins_packed(p, g, bins);
   offset_bins(bins, bin_base);
   gridded += p.keep ? 1u : 0u;
   RecF64 r;
@@ -311,7 +440,61 @@ __device__ __forceinline__ void scatter_rows(
     slot = __shfl_sync(kFull, slot, leader);
     if (bins[s] != kNoBin) {
       slot += __popc(peers & ((1u << lane) - 1u));
-      rec[(uint64_t)bin_off[bins[s]] + slot] = r;
+      store_record(rec + ((uint64_t)bin_off[bins[s]] + slot), r);
+      nrec++;
+    }
+  }
+}
+
+// Pass 2, a lane a row (rows of fewer than eight loads), of the jobs of a batch: the
+// records' places are taken first -- the up to four adds of a row and the bins'
+// offsets are all in flight while its samples are read; one after the other, behind
+// the sums, they were most of the time (26M rows of 2 to 8 samples, 64 jobs: 2.1 ->
+// 1.5 ms).
+template <int N>
+__device__ __forceinline__ void scatter_lane_rows(
+    const double *__restrict__ uu, const double *__restrict__ vv, const double *__restrict__ ww,
+    const float *__restrict__ weight, const float *__restrict__ vis_re,
+    const float *__restrict__ vis_im, uint64_t i, bool valid, uint32_t nchan, uint32_t npol,
+    const Geometry &g, uint32_t bin_base, const uint32_t *__restrict__ bin_off,
+    uint32_t *__restrict__ bin_cursor, RecF64 *__restrict__ rec, uint32_t &gridded,
+    uint32_t &nrec) {
+  const unsigned lane = lane_id();
+  RowPos p;
+  p.keep = false;
+  p.pu = p.pv = 0.0;
+  if (valid) p = row_position(uu[i], vv[i], ww[i], g);
+  uint32_t bins[4], slot[4], off[4];
+  footprint_bins(p, g, bins);
+  const bool need = bins[0] != kNoBin;
+  offset_bins(bins, bin_base);
+  gridded += p.keep ? 1u : 0u;
+#pragma unroll
+  for (int s = 0; s < 4; s++) {
+    slot[s] = off[s] = 0;
+    if (__any_sync(kFull, bins[s] != kNoBin)) {
+      const unsigned peers = __match_any_sync(kFull, bins[s]);
+      if (bins[s] != kNoBin) {
+        if (lane == __ffs(peers) - 1) slot[s] = atomicAdd(&bin_cursor[bins[s]], __popc(peers));
+        off[s] = __ldg(&bin_off[bins[s]]) + __popc(peers & ((1u << lane) - 1u));
+      }
+    }
+  }
+  RecF64 r;
+  r.sre = r.sim = 0.0;
+  if (need) {  // rows that reach no tile never stream their samples
+    const uint32_t nv = nchan * npol;
+    row_sums<N>(weight + i * npol, vis_re + i * nv, vis_im + i * nv, npol, nv, r.sre, r.sim);
+  }
+  r.pu = p.pu;
+  r.pv = p.pv;
+#pragma unroll
+  for (int s = 0; s < 4; s++) {
+    if (!__any_sync(kFull, bins[s] != kNoBin)) continue;
+    const unsigned peers = __match_any_sync(kFull, bins[s]);
+    const uint32_t first = __shfl_sync(kFull, slot[s], __ffs(peers) - 1);
+    if (bins[s] != kNoBin) {
+      store_record(rec + ((uint64_t)off[s] + first), r);
       nrec++;
     }
   }
@@ -329,7 +512,7 @@ __device__ __forceinline__ void add_scatter_counts(uint32_t gridded, uint32_t nr
   }
 }
 
-template <int G, bool V4, bool SHARD>
+template <int G, int N, bool SHARD>
 __global__ void __launch_bounds__(256)
     k_bin_scatter(const double *__restrict__ uu, const double *__restrict__ vv,
                   const double *__restrict__ ww, const float *__restrict__ weight,
@@ -341,17 +524,16 @@ __global__ void __launch_bounds__(256)
   const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
   uint32_t gridded = 0, nrec = 0;
   for (uint64_t base = warp * 32; base < nrows; base += nwarps * 32)
-    scatter_rows<G, V4, SHARD>(uu, vv, ww, weight, vis_re, vis_im, nrows, nchan, npol, g, base,
-                               0, bin_off, bin_cursor, rec, gridded, nrec);
+    scatter_rows<G, N, SHARD>(uu, vv, ww, weight, vis_re, vis_im, nrows, nchan, npol, g, base, 0,
+                              bin_off, bin_cursor, rec, gridded, nrec);
   add_scatter_counts(gridded, nrec, counters);
 }
 
 // The same over the jobs of one sample-pass schedule of a batch (lanes per row
-// G, load width V4): the k-th listed job's rows are units sc_units[k] ..
-// sc_units[k+1]-1 (a unit is 32 rows of one job).  Bounded to three blocks
-// per SM: the job lookup and the per-job geometry add registers to the
-// single-job kernel's set.
-template <int G, bool V4>
+// G, N samples a load): the k-th listed job's rows are units sc_units[k] ..
+// sc_units[k+1]-1 (a unit is 32 rows of one job).  A warp takes a run of units, so
+// that the job lookup is paid once a run.
+template <int G, int N>
 __global__ void __launch_bounds__(256, 3)
     k_bin_scatter_batch(const BatchJob *__restrict__ jobs, const uint32_t *__restrict__ sc_jobs,
                         const uint64_t *__restrict__ sc_units, int lo, int hi,
@@ -360,64 +542,182 @@ __global__ void __launch_bounds__(256, 3)
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
   uint32_t gridded = 0, nrec = 0;
-  const uint64_t u1 = sc_units[hi];
-  for (uint64_t u = sc_units[lo] + warp; u < u1; u += nwarps) {
-    const int k = lo + batch_job_of(sc_units + lo, hi - lo, u);
-    const BatchJob &J = jobs[sc_jobs[k]];
-    const Geometry g = J.g;
-    scatter_rows<G, V4, false>(J.uu, J.vv, J.ww, J.weight, J.vis_re, J.vis_im, J.nrows, J.nchan, J.npol,
-                        g, (u - sc_units[k]) * 32, J.bin_base, bin_off, bin_cursor, rec, gridded,
-                        nrec);
+  const uint64_t first = sc_units[lo];
+  uint64_t u, u1;
+  warp_run(sc_units[hi] - first, warp, nwarps, u, u1);
+  u += first;
+  u1 += first;
+  if (u < u1) {
+    int k = lo + batch_job_of(sc_units + lo, hi - lo, u);
+    while (u < u1) {
+      while (sc_units[k + 1] <= u) k++;
+      const uint64_t j0 = sc_units[k], end = min(u1, sc_units[k + 1]);
+      // the job's fields are read where used, not held in registers
+      const BatchJob &J = jobs[sc_jobs[k]];
+      for (; u < end; u++) {
+        const uint64_t base = (u - j0) * 32;
+        if constexpr (G == 1)
+          scatter_lane_rows<N>(J.uu, J.vv, J.ww, J.weight, J.vis_re, J.vis_im, base + lane_id(),
+                               base + lane_id() < J.nrows, J.nchan, J.npol, J.g, J.bin_base,
+                               bin_off, bin_cursor, rec, gridded, nrec);
+        else
+          scatter_rows<G, N, false>(J.uu, J.vv, J.ww, J.weight, J.vis_re, J.vis_im, J.nrows,
+                                    J.nchan, J.npol, J.g, base, J.bin_base, bin_off, bin_cursor,
+                                    rec, gridded, nrec);
+      }
+    }
   }
   add_scatter_counts(gridded, nrec, counters);
 }
 
-template <int G, bool V4>
-void launch_scatter(int blocks, cudaStream_t st, const double *uu, const double *vv,
-                    const double *ww, const float *weight, const float *vis_re,
-                    const float *vis_im, uint64_t nrows, uint32_t nchan, uint32_t npol,
-                    const Geometry &g, Scratch &s) {
-  RICK_LAUNCHED();
-  if (g.nw_total > 0 && g.nw_total != g.nw)
-    k_bin_scatter<G, V4, true><<<blocks, 256, 0, st>>>(uu, vv, ww, weight, vis_re, vis_im, nrows,
-                                                       nchan, npol, g, s.bin_count, s.bin_cursor,
-                                                       s.records, s.counters);
-  else
-    k_bin_scatter<G, V4, false><<<blocks, 256, 0, st>>>(uu, vv, ww, weight, vis_re, vis_im, nrows,
-                                                        nchan, npol, g, s.bin_count, s.bin_cursor,
-                                                        s.records, s.counters);
+// Pass 2, a lane a row (rows of fewer than eight loads), of one job: the records'
+// places are taken block by block.  The uv centre is dense, so with places taken
+// warp by warp its bins' cursors took an add from nearly every warp, one after
+// another at one address (280k rows of 16 samples: 52 us; 31 here); the warps of a
+// block add up in a shared table first, and the block adds each bin once -- while
+// the samples are read.  A bin whose slots of the table are taken gets its places
+// from the cursor directly.
+constexpr int kShortThreads = 512;
+constexpr int kPlaceSlots = 1024;
+__device__ __forceinline__ uint32_t place_slot(uint32_t bin) {
+  return (bin * 2654435761u) >> (32 - 10);
+}
+struct __align__(16) PlaceTable {
+  uint32_t key[kPlaceSlots], cnt[kPlaceSlots], at[kPlaceSlots];
+};
+
+template <int N>
+__global__ void __launch_bounds__(kShortThreads, 2)
+    k_bin_scatter_short(const double *__restrict__ uu, const double *__restrict__ vv,
+                        const double *__restrict__ ww, const float *__restrict__ weight,
+                        const float *__restrict__ vis_re, const float *__restrict__ vis_im,
+                        uint64_t nrows, uint32_t nchan, uint32_t npol, Geometry g,
+                        const uint32_t *__restrict__ bin_off, uint32_t *__restrict__ bin_cursor,
+                        RecF64 *__restrict__ rec, uint64_t *__restrict__ counters) {
+  __shared__ PlaceTable place_table;
+  PlaceTable *table = &place_table;
+  const unsigned lane = lane_id();
+  uint32_t gridded = 0, nrec = 0;
+  for (uint64_t base = blockIdx.x * (uint64_t)kShortThreads; base < nrows;
+       base += gridDim.x * (uint64_t)kShortThreads) {
+    const uint64_t i = base + threadIdx.x;
+    if (threadIdx.x < kPlaceSlots / 4) {
+      reinterpret_cast<uint4 *>(table->key)[threadIdx.x] = make_uint4(kNoBin, kNoBin, kNoBin, kNoBin);
+      reinterpret_cast<uint4 *>(table->cnt)[threadIdx.x] = make_uint4(0, 0, 0, 0);
+    }
+    RowPos p;
+    p.keep = false;
+    p.pu = p.pv = 0.0;
+    if (i < nrows) p = row_position(__ldg(uu + i), __ldg(vv + i), __ldg(ww + i), g);
+    uint32_t bins[4];
+    footprint_bins(p, g, bins);
+    const bool need = bins[0] != kNoBin;
+    gridded += p.keep ? 1u : 0u;
+    __syncthreads();  // the table is clear
+    // Of the lanes with one bin the first adds for all.  place[s], on that lane: the
+    // table slot and the rank so far (bit s of `in_table`), or the first place itself;
+    // nobody waits for it before the records are written.
+    uint32_t place[4], who[4], in_table = 0;
+#pragma unroll
+    for (int s = 0; s < 4; s++) {
+      place[s] = who[s] = 0;
+      if (!__any_sync(kFull, bins[s] != kNoBin)) continue;
+      const unsigned peers = __match_any_sync(kFull, bins[s]);
+      const unsigned leader = __ffs(peers) - 1;
+      who[s] = leader | (uint32_t)__popc(peers & ((1u << lane) - 1u)) << 8;
+      if (bins[s] != kNoBin && lane == leader) {
+        const uint32_t n = __popc(peers);
+        uint32_t h = place_slot(bins[s]);
+        bool mine = false;
+#pragma unroll
+        for (int probe = 0; probe < 2 && !mine; probe++) {
+          h ^= probe;  // the slot, then its neighbour
+          uint32_t k = *(volatile uint32_t *)&table->key[h];
+          if (k == kNoBin) k = atomicCAS(&table->key[h], kNoBin, bins[s]);
+          mine = k == kNoBin || k == bins[s];
+        }
+        if (mine) {
+          in_table |= 1u << s;
+          place[s] = h << 16 | atomicAdd(&table->cnt[h], n);
+        } else {
+          place[s] = __ldg(&bin_off[bins[s]]) + atomicAdd(&bin_cursor[bins[s]], n);
+        }
+      }
+    }
+    __syncthreads();  // the block's counts are complete
+#pragma unroll
+    for (int k = threadIdx.x; k < kPlaceSlots; k += kShortThreads) {
+      const uint32_t n = table->cnt[k];
+      if (n) {
+        const uint32_t bin = table->key[k];
+        table->at[k] = __ldg(&bin_off[bin]) + atomicAdd(&bin_cursor[bin], n);
+      }
+    }
+    RecF64 r;
+    r.sre = r.sim = 0.0;
+    if (need) {  // rows that reach no tile (other shards') never stream their samples
+      const uint32_t nv = nchan * npol;
+      row_sums<N>(weight + i * npol, vis_re + i * nv, vis_im + i * nv, npol, nv, r.sre, r.sim);
+    }
+    r.pu = p.pu;
+    r.pv = p.pv;
+    __syncthreads();  // the places are known
+#pragma unroll
+    for (int s = 0; s < 4; s++) {
+      if (!__any_sync(kFull, bins[s] != kNoBin)) continue;
+      const uint32_t first = __shfl_sync(kFull, place[s], who[s] & 31u);
+      const uint32_t tab = __shfl_sync(kFull, in_table, who[s] & 31u) >> s & 1u;
+      if (bins[s] == kNoBin) continue;
+      const uint32_t at = (tab ? table->at[first >> 16] + (first & 0xffffu) : first) + (who[s] >> 8);
+      store_record(rec + at, r);
+      nrec++;
+    }
+    __syncthreads();  // the table is cleared for the next rows
+  }
+  add_scatter_counts(gridded, nrec, counters);
 }
 
 }  // namespace
-
-int lanes_per_row(uint64_t per_row);
 
 // Pass 1 and the offsets: histogram of records per bin over all rows, bin
 // offsets and work-item offsets (records are not written yet).
 int bin_count_rows(const Geometry &g, uint64_t nrows, const double *uu, const double *vv,
                    const double *ww, Scratch &s, uint32_t max_chunk, cudaStream_t st) {
   const uint64_t nbins = g.nbins();
-  RICK_CUDA(cudaMemsetAsync(s.bin_count, 0, (nbins + 1) * sizeof(uint32_t), st));
-  RICK_CUDA(cudaMemsetAsync(s.bin_cursor, 0, nbins * sizeof(uint32_t), st));
   if (nrows == 0) {
     RICK_CUDA(cudaMemsetAsync(s.item_off, 0, (nbins + 1) * sizeof(uint32_t), st));
     return RICK_OK;
   }
-  const int sms = num_sms();
-  const uint64_t warps_needed = (nrows + 31) / 32;
-  const int blocks_cnt = (int)std::min<uint64_t>((warps_needed + 7) / 8, (uint64_t)sms * 16);
+  // four units a warp where there are few: a block's cache costs its clearing and
+  // its flush
+  const uint64_t warps = ((nrows + 31) / 32 + kCountUnits - 1) / kCountUnits;
+  const int blocks = (int)std::min<uint64_t>((warps + 7) / 8, (uint64_t)num_sms() * 8);
   RICK_LAUNCHED();
-  k_bin_count<<<blocks_cnt, 256, 0, st>>>(uu, vv, ww, nrows, g, s.bin_count, s.counters);
+  k_bin_count<<<blocks, 256, 0, st>>>(uu, vv, ww, nrows, g, s.bin_count, s.counters);
   RICK_CUDA(cudaGetLastError());
-  // counts -> exclusive offsets, in place (bin_count[nbins] becomes the total)
-  RICK_TRY(exclusive_scan_u32(s.bin_count, s.bin_count, nbins + 1, s.scan_tmp, st));
-  // work items
-  const int blocks_items = (int)std::min<uint64_t>((nbins + 256) / 256, (uint64_t)sms * 32);
-  RICK_LAUNCHED();
-  k_item_count<<<blocks_items, 256, 0, st>>>(s.bin_count, nbins, max_chunk, s.item_off);
-  RICK_CUDA(cudaGetLastError());
-  RICK_TRY(exclusive_scan_u32(s.item_off, s.item_off, nbins + 1, s.scan_tmp, st));
-  return RICK_OK;
+  return scan_bins(s.bin_count, s.item_off, nbins, max_chunk, s.scan_tmp, st);
+}
+
+// Lanes that share one row's samples: one for rows of fewer than eight loads (a row
+// spread over lanes would leave each lane a load or two and the warp waiting), four
+// up to fifteen, then enough to cover the row's loads in one or two sweeps.  A shard
+// that holds less than half of the planes reads rows of eight loads a lane a row: it
+// skips rows one by one (2.8M of 3.8M rows: 0.32 ms against 0.35 with four lanes).
+int lanes_per_row(uint64_t per_row, bool skips) {
+  if (per_row < 8 || (skips && per_row == 8)) return 1;
+  if (per_row < 16) return skips ? 8 : 4;
+  int G = 16;
+  while (G < 32 && (uint64_t)G * 2 <= per_row) G *= 2;
+  return G;
+}
+
+// 16-byte loads where the rows start on 16 bytes and a load's polarisations repeat
+// row by row; else 8-byte loads of pairs on the same terms.
+int sample_vector(const float *vis_re, const float *vis_im, uint64_t nv, uint32_t npol) {
+  const uintptr_t at = (uintptr_t)vis_re | (uintptr_t)vis_im;
+  if (at % 16 == 0 && nv % 4 == 0 && (npol == 1 || npol == 2 || npol == 4)) return 4;
+  if (at % 8 == 0 && nv % 2 == 0 && (npol == 1 || npol == 2)) return 2;
+  return 1;
 }
 
 // Pass 2 over rows [0, nrows) of the arrays given (a contiguous slice of the
@@ -428,104 +728,70 @@ int bin_scatter_rows(const Geometry &g, uint64_t nrows, const double *uu, const 
                      const float *vis_im, uint32_t nchan, uint32_t npol, Scratch &s,
                      cudaStream_t st) {
   if (nrows == 0) return RICK_OK;
-  const int sms = num_sms();
-  const uint64_t warps_needed = (nrows + 31) / 32;
   const uint64_t nv = (uint64_t)nchan * npol;
-  const bool aligned = ((uintptr_t)vis_re % 16 == 0) && ((uintptr_t)vis_im % 16 == 0);
-  const bool v4 = aligned && nv % 4 == 0 && (npol == 1 || npol == 2 || npol == 4);
-  const uint64_t per_row = v4 ? nv / 4 : nv;
-  // lanes per row: enough to cover a row's 16-byte chunks in one or two sweeps
-  const int G = lanes_per_row(per_row);
-  const int blocks = (int)std::min<uint64_t>((warps_needed + 7) / 8, (uint64_t)sms * 8);
-#define RICK_SCATTER(GG)                                                                    \
-  case GG:                                                                                  \
-    if (v4)                                                                                 \
-      launch_scatter<GG, true>(blocks, st, uu, vv, ww, weight, vis_re, vis_im, nrows, nchan, \
-                               npol, g, s);                                                 \
-    else                                                                                    \
-      launch_scatter<GG, false>(blocks, st, uu, vv, ww, weight, vis_re, vis_im, nrows,      \
-                                nchan, npol, g, s);                                         \
-    break;
-  switch (G) {
-    RICK_SCATTER(1)
-    RICK_SCATTER(2)
-    RICK_SCATTER(4)
-    RICK_SCATTER(8)
-    RICK_SCATTER(16)
-    RICK_SCATTER(32)
+  const int N = sample_vector(vis_re, vis_im, nv, npol);
+  const int sms = num_sms();
+  const bool skips = g.nw_total > 0 && 2 * g.nw < g.nw_total;
+  const int G = lanes_per_row(nv / N, skips);
+  RICK_LAUNCHED();
+  if (G == 1 && !skips) {
+    const uint64_t need = (nrows + kShortThreads - 1) / kShortThreads;
+    const int blocks = (int)std::min<uint64_t>(need, (uint64_t)sms * 2);
+#define RICK_SHORT(NN)                                                                          \
+  if (N == NN)                                                                                  \
+    k_bin_scatter_short<NN><<<blocks, kShortThreads, 0, st>>>(                                  \
+        uu, vv, ww, weight, vis_re, vis_im, nrows, nchan, npol, g, s.bin_count, s.bin_cursor,   \
+        s.records, s.counters);
+    RICK_SHORT(4) RICK_SHORT(2) RICK_SHORT(1)
+#undef RICK_SHORT
+    RICK_CUDA(cudaGetLastError());
+    return RICK_OK;
   }
-#undef RICK_SCATTER
+  const int blocks = (int)std::min<uint64_t>(((nrows + 31) / 32 + 7) / 8, (uint64_t)sms * 8);
+#define RICK_LONG(GG, NN)                                                                        \
+  if (G == GG && N == NN) {                                                                      \
+    if (skips)                                                                                   \
+      k_bin_scatter<GG, NN, true><<<blocks, 256, 0, st>>>(uu, vv, ww, weight, vis_re, vis_im,    \
+                                                          nrows, nchan, npol, g, s.bin_count,    \
+                                                          s.bin_cursor, s.records, s.counters);  \
+    else                                                                                         \
+      k_bin_scatter<GG, NN, false><<<blocks, 256, 0, st>>>(uu, vv, ww, weight, vis_re, vis_im,   \
+                                                           nrows, nchan, npol, g, s.bin_count,   \
+                                                           s.bin_cursor, s.records, s.counters); \
+  }
+#define RICK_LANES(X, NN) X(1, NN) X(4, NN) X(8, NN) X(16, NN) X(32, NN)
+  RICK_LANES(RICK_LONG, 4) RICK_LANES(RICK_LONG, 2) RICK_LANES(RICK_LONG, 1)
+#undef RICK_LONG
   RICK_CUDA(cudaGetLastError());
   return RICK_OK;
 }
 
-int bin_rows(const Geometry &g, int kernel, int precision, uint64_t nrows, const double *uu,
-             const double *vv, const double *ww, const float *weight, const float *vis_re,
-             const float *vis_im, uint32_t nchan, uint32_t npol, Scratch &s,
-             uint32_t max_chunk, cudaStream_t st, cudaEvent_t mid) {
-  (void)kernel;
-  (void)precision;
-  RICK_TRY(bin_count_rows(g, nrows, uu, vv, ww, s, max_chunk, st));
-  if (mid) RICK_CUDA(cudaEventRecord(mid, st));
-  return bin_scatter_rows(g, nrows, uu, vv, ww, weight, vis_re, vis_im, nchan, npol, s, st);
-}
-
-// Lanes that share one row's samples: enough to cover the row's loads in one
-// or two sweeps; rows of at most 8 loads are read by one lane each (a row
-// spread over lanes would leave each lane one load and the warp waiting).
-int lanes_per_row(uint64_t per_row) {
-  if (per_row <= 8) return 1;
-  int G = 1;
-  while (G < 32 && (uint64_t)G * 2 <= per_row) G *= 2;
-  return G;
-}
-
 int bin_rows_batch(const BatchLaunch &b, Scratch &s, uint32_t max_chunk, cudaStream_t st) {
   const uint64_t nbins = b.total_bins;
-  RICK_CUDA(cudaMemsetAsync(s.bin_count, 0, (nbins + 1) * sizeof(uint32_t), st));
-  RICK_CUDA(cudaMemsetAsync(s.bin_cursor, 0, std::max<uint64_t>(nbins, 1) * sizeof(uint32_t), st));
   const int sms = num_sms();
   const uint64_t units = b.total_row_units;
-  const int blocks_cnt = (int)std::max<uint64_t>(1, std::min<uint64_t>((units + 7) / 8, (uint64_t)sms * 16));
+  const uint64_t warps = (units + kCountUnits - 1) / kCountUnits;
+  const int blocks_cnt =
+      (int)std::max<uint64_t>(1, std::min<uint64_t>((warps + 7) / 8, (uint64_t)sms * 8));
   RICK_LAUNCHED();
   k_bin_count_batch<<<blocks_cnt, 256, 0, st>>>(b.jobs, b.njobs, b.u.row_units, units,
                                                 s.bin_count, s.counters);
   RICK_CUDA(cudaGetLastError());
-  RICK_TRY(exclusive_scan_u32(s.bin_count, s.bin_count, nbins + 1, s.scan_tmp, st));
-  const int blocks_items = (int)std::min<uint64_t>((nbins + 256) / 256, (uint64_t)sms * 32);
-  RICK_LAUNCHED();
-  k_item_count<<<blocks_items, 256, 0, st>>>(s.bin_count, nbins, max_chunk, s.item_off);
-  RICK_CUDA(cudaGetLastError());
-  RICK_TRY(exclusive_scan_u32(s.item_off, s.item_off, nbins + 1, s.scan_tmp, st));
+  RICK_TRY(scan_bins(s.bin_count, s.item_off, nbins, max_chunk, s.scan_tmp, st));
   for (int c = 0; c < b.n_sc; c++) {
     const ScatterClass &k = b.sc[c];
     const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>((k.units + 7) / 8,
-                                                                      (uint64_t)sms * 8));
-#define RICK_SC(GG)                                                                            \
-  case GG:                                                                                     \
-    RICK_LAUNCHED();                                                                           \
-    if (k.v4)                                                                                  \
-      k_bin_scatter_batch<GG, true><<<blocks, 256, 0, st>>>(b.jobs, b.sc_jobs, b.sc_units, k.lo, \
-                                                            k.hi, s.bin_count, s.bin_cursor,    \
-                                                            s.records, s.counters);             \
-    else                                                                                       \
-      k_bin_scatter_batch<GG, false><<<blocks, 256, 0, st>>>(b.jobs, b.sc_jobs, b.sc_units,     \
-                                                             k.lo, k.hi, s.bin_count,           \
-                                                             s.bin_cursor, s.records,           \
-                                                             s.counters);                       \
-    break;
-    switch (k.lanes) {
-      RICK_SC(1)
-      RICK_SC(2)
-      RICK_SC(4)
-      RICK_SC(8)
-      RICK_SC(16)
-      RICK_SC(32)
-    }
+                                                                      (uint64_t)sms * 6));
+    RICK_LAUNCHED();
+#define RICK_SC(GG, NN)                                                                      \
+  if (k.lanes == GG && k.vec == NN)                                                          \
+    k_bin_scatter_batch<GG, NN><<<blocks, 256, 0, st>>>(b.jobs, b.sc_jobs, b.sc_units, k.lo, \
+                                                        k.hi, s.bin_count, s.bin_cursor,     \
+                                                        s.records, s.counters);
+    RICK_LANES(RICK_SC, 4) RICK_LANES(RICK_SC, 2) RICK_LANES(RICK_SC, 1)
 #undef RICK_SC
     RICK_CUDA(cudaGetLastError());
   }
-  RICK_CUDA(cudaGetLastError());
   return RICK_OK;
 }
 

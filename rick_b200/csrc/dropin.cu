@@ -364,12 +364,12 @@ int rick_host_free(void *ptr) {
 }
 
 int rick_kernel_names(const char **names, int max_names) {
-  static const char *k[] = {"k_bin_count",        "k_item_count",       "k_bin_scatter",
-                            "k_scan_block",       "k_scan_add",         "k_grid_tiles",
+  static const char *k[] = {"k_bin_count",        "k_scan_sums",        "k_scan_bins",
+                            "k_bin_scatter",      "k_grid_tiles",
                             "k_zero_split_tiles", "k_row_list",         "k_fft_units",
                             "k_fft_rows",         "k_fft_cols",         "k_phase_sum",
                             "k_export_cube",      "k_import_cube",      "k_bin_count_batch",
-                            "k_bin_scatter_batch", "k_grid_tiles_batch", "k_zero_split_tiles_batch",
+                            "k_bin_scatter_batch", "k_bin_scatter_short", "k_grid_tiles_batch", "k_zero_split_tiles_batch",
                             "k_fft_rows_multi",   "k_fft_cols_multi",   "k_uvw_init",
                             "k_uvw_extrema",      "k_uvw_normalize"};
   const int n = (int)(sizeof(k) / sizeof(k[0]));

@@ -734,9 +734,10 @@ __global__ void __launch_bounds__(Shape<L>::kThreads, col_blocks<S, L>())
 // plane w (at the job's counts_base).  The mask itself is turned for the column
 // pass: bit r of 16-bit entry t of a plane is row t + G r (G = ny / 16; for
 // ny = 8192 the halves of the plane apart, G = 256), what thread t loads.  Clears
-// the image (clear_n pixels) for a column pass that adds to it.
-__global__ void k_row_list(const BatchJob *__restrict__ jobs, int njobs,
-                           const uint64_t *__restrict__ mask_base, uint64_t nwords,
+// the image (clear_n pixels) for a column pass that adds to it.  A plan's job comes
+// as a parameter (jobs null).
+__global__ void k_row_list(const BatchJob *__restrict__ jobs, const __grid_constant__ BatchJob one,
+                           int njobs, const uint64_t *__restrict__ mask_base, uint64_t nwords,
                            const uint32_t *__restrict__ rowmask, uint32_t *__restrict__ rowlist,
                            uint32_t *__restrict__ counts, uint16_t *__restrict__ rowbits,
                            double *__restrict__ clear_re, double *__restrict__ clear_im,
@@ -747,8 +748,7 @@ __global__ void k_row_list(const BatchJob *__restrict__ jobs, int njobs,
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nwords;
        i += gridDim.x * (uint64_t)blockDim.x) {
     uint32_t bits = rowmask[i];
-    const int j = batch_job_of(mask_base, njobs, i);
-    const BatchJob &J = jobs[j];
+    const BatchJob &J = jobs ? jobs[batch_job_of(mask_base, njobs, i)] : one;
     const uint64_t li = i - J.mask_base;
     const uint32_t nty = (uint32_t)J.g.nty, ny = (uint32_t)J.g.ny;
     const uint32_t w = (uint32_t)(li / nty), band = (uint32_t)(li % nty);
@@ -973,14 +973,13 @@ void fft_classes(const BatchJob *jobs, int njobs, int precision, FftJobs &f, uin
 }
 
 int sparse_fft_lists(const FftJobs &f, int precision, cudaStream_t st) {
-  RICK_CUDA(cudaMemsetAsync(f.counts, 0, sizeof(uint32_t) * f.total_count_words, st));
   const uint64_t nwords = f.total_mask_words;
   const uint64_t clear = f.one && f.cols_parts > 1 ? (uint64_t)f.one->g.nx * f.one->g.ny : 0;
   const int blocks = (int)std::min<uint64_t>((std::max(nwords, clear / 8) + 255) / 256,
                                              (uint64_t)num_sms() * 8);
   RICK_LAUNCHED();
   k_row_list<<<std::max(blocks, 1), 256, 0, st>>>(
-      f.jobs, f.njobs, f.mask_base, nwords, f.rowmask, f.rowlist, f.counts, f.rowbits,
+      f.one ? nullptr : f.jobs, f.one ? *f.one : BatchJob{}, f.njobs, f.mask_base, nwords, f.rowmask, f.rowlist, f.counts, f.rowbits,
       clear ? f.one->img_re : nullptr, clear ? f.one->img_im : nullptr, clear);
   RICK_CUDA(cudaGetLastError());
   if (!f.one) {  // one job's row pass reads its row count directly

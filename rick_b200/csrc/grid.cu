@@ -393,29 +393,43 @@ __device__ __forceinline__ void zero_tile(const Geometry &g, uint64_t b,
   }
 }
 
+// Bins with more than one work item: zero(b) runs for each by a whole warp.  A warp
+// looks at up to 32 neighbouring bins at a time (a lane each), at fewer where there
+// are fewer bins: split tiles are neighbours at the uv centre, and one warp should
+// not clear them all.
+template <typename Zero>
+__device__ __forceinline__ void for_split_bins(const uint32_t *__restrict__ item_off, uint32_t nbins,
+                                               Zero zero) {
+  const unsigned lane = threadIdx.x & 31u;
+  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
+  const uint32_t per = (uint32_t)min((uint64_t)32, max((uint64_t)1, nbins / nwarps));
+  for (uint64_t b0 = warp * per; b0 < nbins; b0 += nwarps * per) {
+    const uint64_t b = b0 + lane;
+    unsigned split =
+        __ballot_sync(kFull, lane < per && b < nbins && item_off[b + 1] - item_off[b] > 1);
+    while (split) {
+      zero((uint32_t)b0 + __ffs(split) - 1);
+      split &= split - 1;
+    }
+  }
+}
+
 template <typename OutT>
 __global__ void k_zero_split_tiles(const uint32_t *__restrict__ item_off, uint32_t nbins, Geometry g,
                                    typename Vec2<OutT>::type *__restrict__ cube) {
-  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
-  for (uint64_t b = warp; b < nbins; b += nwarps) {
-    if (item_off[b + 1] - item_off[b] <= 1) continue;
-    zero_tile<OutT>(g, b, cube);
-  }
+  for_split_bins(item_off, nbins, [&](uint32_t b) { zero_tile<OutT>(g, b, cube); });
 }
 
 template <typename OutT>
 __global__ void k_zero_split_tiles_batch(const BatchJob *__restrict__ jobs, int njobs,
                                          const uint32_t *__restrict__ bin_base,
                                          const uint32_t *__restrict__ item_off, uint32_t nbins) {
-  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
-  for (uint64_t b = warp; b < nbins; b += nwarps) {
-    if (item_off[b + 1] - item_off[b] <= 1) continue;
-    const int j = batch_job_of(bin_base, njobs, (uint32_t)b);
+  for_split_bins(item_off, nbins, [&](uint32_t b) {
+    const int j = batch_job_of(bin_base, njobs, b);
     const Geometry g = jobs[j].g;
     zero_tile<OutT>(g, b - jobs[j].bin_base, (typename Vec2<OutT>::type *)jobs[j].cube);
-  }
+  });
 }
 
 template <typename OutT>
@@ -458,8 +472,7 @@ int grid_tiles(const Geometry &g, int kernel, int precision, Scratch &s, void *c
 
 int zero_split_tiles(const Geometry &g, int precision, Scratch &s, void *cube, cudaStream_t st) {
   const uint32_t nbins = (uint32_t)g.nbins();
-  const int blocks = (int)std::min<uint64_t>(((uint64_t)nbins * 32 + 255) / 256,
-                                             (uint64_t)num_sms() * 16);
+  const int blocks = (int)std::min<uint64_t>(((uint64_t)nbins * 32 + 255) / 256, (uint64_t)num_sms() * 8);
   RICK_LAUNCHED();
   if (precision == RICK_PREC_FP64)
     k_zero_split_tiles<double><<<std::max(blocks, 1), 256, 0, st>>>(s.item_off, nbins, g,
@@ -477,7 +490,7 @@ template <typename OutT>
 int launch_grid_batch(const BatchLaunch &b, Scratch &s, uint32_t max_chunk, cudaStream_t st) {
   const int sms = num_sms();
   const uint32_t nbins = b.total_bins;
-  const int zblocks = (int)std::min<uint64_t>(((uint64_t)nbins * 32 + 255) / 256, (uint64_t)sms * 16);
+  const int zblocks = (int)std::min<uint64_t>(((uint64_t)nbins * 32 + 255) / 256, (uint64_t)sms * 8);
   RICK_LAUNCHED();
   k_zero_split_tiles_batch<OutT><<<std::max(zblocks, 1), 256, 0, st>>>(b.jobs, b.njobs,
                                                                       b.u.bin_base, s.item_off,

@@ -153,8 +153,7 @@ int rick_wstack_noalloc(int num_w_planes, uint64_t num_points, uint32_t freq_per
   g.half = (w_support - 1) / 2;
   g.ntx = (g.nx + kTile - 1) / kTile;
   g.nty = (g.ny + kTile - 1) / kTile;
-  g.dx = dx;
-  g.dw = dw;
+  g.set_spacing(dx, dw);
   g.w_supporth = (double)g.half * (1.0 / (double)g.nx);
   g.select_sector0 = 0;
   const uint64_t tiles = (uint64_t)g.ntx * (uint64_t)g.nty;  // < 2^52
@@ -185,13 +184,16 @@ int rick_wstack_noalloc(int num_w_planes, uint64_t num_points, uint32_t freq_per
   s.scan_tmp = (uint32_t *)(b + L.scan_tmp);
   s.records = (RecF64 *)(b + L.records);
   s.max_records = 4 * num_points;
-  // what must start at zero: the counters (bin counts and cursors are cleared
-  // by bin_rows itself), and the caller's cube (overwrite semantics)
+  // what must start at zero: the counters, the bin counts and cursors, and the
+  // caller's cube (overwrite semantics)
   RICK_CUDA(cudaMemsetAsync(s.counters, 0, kNumCounters * sizeof(uint64_t), st));
+  RICK_CUDA(cudaMemsetAsync(s.bin_count, 0, (nbins + 1) * sizeof(uint32_t), st));
+  RICK_CUDA(cudaMemsetAsync(s.bin_cursor, 0, nbins * sizeof(uint32_t), st));
   const uint64_t per = num_points / ((uint64_t)num_sms() * 4 + 1);
   const uint32_t chunk = (uint32_t)(per < 1024 ? 1024 : (per > 8192 ? 8192 : per));
-  RICK_TRY(bin_rows(g, kernel, RICK_PREC_FP64, num_points, uu, vv, ww, weight, vis_real, vis_img,
-                    freq_per_chan, polarizations, s, chunk, st));
+  RICK_TRY(bin_count_rows(g, num_points, uu, vv, ww, s, chunk, st));
+  RICK_TRY(bin_scatter_rows(g, num_points, uu, vv, ww, weight, vis_real, vis_img, freq_per_chan,
+                            polarizations, s, st));
   RICK_CUDA(cudaMemsetAsync(grid, 0, 2ull * num_w_planes * grid_size_x * grid_size_y * 8, st));
   RICK_TRY(grid_tiles(g, kernel, RICK_PREC_FP64, s, grid, 0, chunk, st));
   return RICK_OK;

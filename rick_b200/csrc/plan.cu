@@ -158,9 +158,10 @@ struct rick_plan {
   bool sparse = false;
   FftScratch f{};
   FftJobs fj{};
-  BatchJob *d_job = nullptr;      // [1]
-  uint32_t *d_fft_tabs = nullptr; // fft_units [2], col_jobs [1], col_units [2]
-  uint64_t *d_mask_base = nullptr;  // [2]
+  // cleared together before every gridding: counters, bin counts and cursors, and
+  // (sparse) the row and tile masks and the row counts
+  char *d_clear = nullptr;
+  size_t clear_bytes = 0;
 };
 
 namespace {
@@ -222,8 +223,7 @@ void fill_geometry(rick_plan *p, double dx, double dw, int select) {
   g.half = (p->d.w_support - 1) / 2;
   g.ntx = (g.nx + kTile - 1) / kTile;
   g.nty = (g.ny + kTile - 1) / kTile;
-  g.dx = dx;
-  g.dw = dw;
+  g.set_spacing(dx, dw);
   g.w_supporth = (double)g.half * (1.0 / (double)g.nx);  // init.c:13 uses the global dx
   g.select_sector0 = select;
 }
@@ -341,7 +341,7 @@ int grid_begin(rick_plan *p, uint64_t nrows, const double *uu, const double *vv,
   if (p->d.normalize_uvw && nrows)  // gridding.c:21-83, in place
     RICK_TRY(normalize_uvw(nrows, const_cast<double *>(uu), const_cast<double *>(vv),
                            const_cast<double *>(ww), p->d_norm, st));
-  RICK_CUDA(cudaMemsetAsync(p->s.counters, 0, kNumCounters * sizeof(uint64_t), st));
+  RICK_CUDA(cudaMemsetAsync(p->d_clear, 0, p->clear_bytes, st));
   p->chunk = choose_chunk(nrows);
   RICK_TRY(bin_count_rows(p->g, nrows, uu, vv, ww, p->s, p->chunk, st));
   return mark(p, p->ev[1], st);
@@ -357,11 +357,7 @@ int grid_samples(rick_plan *p, uint64_t nrows, const double *uu, const double *v
 int grid_finish(rick_plan *p, uint64_t nrows, int accumulate, bool sparse, cudaStream_t st) {
   RICK_TRY(mark(p, p->ev[2], st));
   if (sparse) {
-    // only the tiles several work items add into are cleared; the row mask
-    // records which grid rows the footprints reach
-    RICK_CUDA(cudaMemsetAsync(p->f.rowmask, 0, (size_t)p->g.nw * p->g.nty * 4, st));
-    RICK_CUDA(cudaMemsetAsync(p->f.tilemask, 0,
-                              (size_t)p->g.nw * p->g.nty * ((p->g.ntx + 31) / 32) * 4, st));
+    // only the tiles several work items add into are cleared
     RICK_TRY(zero_split_tiles(p->g, p->d.precision, p->s, p->cube, st));
   } else if (!accumulate) {
     RICK_CUDA(cudaMemsetAsync(p->cube, 0, p->cube_vals * p->val_bytes, st));
@@ -403,8 +399,6 @@ int image_sparse_after_grid(rick_plan *p, uint64_t nrows, double resolution, dou
   j.phase_on = p->d.phase_on;
   j.img_re = img_re;
   j.img_im = img_im;
-  // from pageable memory: the call returns once `j` has been staged
-  RICK_CUDA(cudaMemcpyAsync(p->d_job, &j, sizeof(j), cudaMemcpyHostToDevice, st));
   p->fj.one = &j;
   RICK_TRY(sparse_fft_lists(p->fj, p->d.precision, st));
   RICK_TRY(sparse_fft_rows(p->fj, p->d.precision, st));
@@ -520,11 +514,8 @@ int rick_plan_create(rick_plan **out, const rick_plan_desc *desc) {
   };
   A(&p->cube, p->cube_vals * p->val_bytes);
   if (desc->normalize_uvw) A(&p->d_norm, RICK_NORMALIZE_SCRATCH);
-  A((void **)&p->s.bin_count, (nbins + 1) * 4);
-  A((void **)&p->s.bin_cursor, nbins * 4);
   A((void **)&p->s.item_off, (nbins + 1) * 4);
   A((void **)&p->s.scan_tmp, scan_tmp_words(nbins + 1) * 4);
-  A((void **)&p->s.counters, kNumCounters * 8);
   p->s.max_records = 4 * std::max<uint64_t>(desc->max_rows, 1);
   A((void **)&p->s.records, p->s.max_records * sizeof(RecF64));
   A((void **)&p->s.table, kIncreasePrecision * kMaxSupport * 8);
@@ -542,13 +533,29 @@ int rick_plan_create(rick_plan **out, const rick_plan_desc *desc) {
   }
   p->sparse = sparse_fft_supported(desc->grid_size_x, desc->grid_size_y) &&
               getenv("RICK_DENSE_FFT") == nullptr;
+  {
+    const size_t masks = (size_t)nwl * p->g.nty, tiles = masks * ((p->g.ntx + 31) / 32);
+    const struct {
+      void **ptr;
+      size_t bytes;
+    } part[] = {{(void **)&p->s.counters, kNumCounters * 8},
+                {(void **)&p->s.bin_count, (nbins + 1) * 4},
+                {(void **)&p->s.bin_cursor, nbins * 4},
+                {(void **)&p->f.rowmask, p->sparse ? masks * 4 : 0},
+                {(void **)&p->f.tilemask, p->sparse ? tiles * 4 : 0},
+                {(void **)&p->f.counts, p->sparse ? (size_t)(1 + nwl) * 4 : 0}};
+    for (const auto &q : part) p->clear_bytes += (q.bytes + 15) & ~(size_t)15;
+    A((void **)&p->d_clear, p->clear_bytes);
+    size_t at = 0;
+    for (const auto &q : part) {
+      if (p->d_clear && q.bytes) *q.ptr = p->d_clear + at;
+      at += (q.bytes + 15) & ~(size_t)15;
+    }
+  }
   if (st == RICK_OK && p->sparse) {
     const int nx = desc->grid_size_x, ny = desc->grid_size_y;
-    A((void **)&p->f.rowmask, (size_t)nwl * p->g.nty * 4);
     A((void **)&p->f.rowbits, (size_t)nwl * p->g.nty * 4);
     A((void **)&p->f.rowlist, (size_t)nwl * ny * 4);
-    A((void **)&p->f.counts, (size_t)(1 + nwl) * 4);
-    A((void **)&p->f.tilemask, (size_t)nwl * p->g.nty * ((p->g.ntx + 31) / 32) * 4);
     A(&p->f.tw_x, twiddle_bytes(nx, desc->precision));
     A(&p->f.tw_y, twiddle_bytes(ny, desc->precision));
     A(&p->f.blocked, p->cube_vals * p->val_bytes);
@@ -568,32 +575,19 @@ int rick_plan_create(rick_plan **out, const rick_plan_desc *desc) {
         free(tab);
       }
     }
-    A((void **)&p->d_job, sizeof(BatchJob));
-    A((void **)&p->d_fft_tabs, 8 * sizeof(uint32_t));
-    A((void **)&p->d_mask_base, 2 * sizeof(uint64_t));
     if (st == RICK_OK) {
       FftJobs &fj = p->fj;
       BatchJob hj = plan_job(p);
-      uint32_t tabs[8] = {};
-      fft_classes(&hj, 1, desc->precision, fj, tabs + 2, tabs + 3);
-      const uint64_t mb[2] = {0, (uint64_t)nwl * p->g.nty};
-      fj.jobs = p->d_job;
+      uint32_t col_job[1], col_units[2];
+      fft_classes(&hj, 1, desc->precision, fj, col_job, col_units);
       fj.njobs = 1;
-      fj.fft_units = p->d_fft_tabs;
-      fj.col_jobs = p->d_fft_tabs + 2;
-      fj.col_units = p->d_fft_tabs + 3;
-      fj.mask_base = p->d_mask_base;
-      fj.total_mask_words = mb[1];
-      fj.total_count_words = 1 + nwl;
+      fj.total_mask_words = (uint64_t)nwl * p->g.nty;
       fj.cols_parts = column_parts(desc->precision, nx, ny, nwl);
       fj.rowmask = p->f.rowmask;
       fj.tilemask = p->f.tilemask;
       fj.rowbits = p->f.rowbits;
       fj.rowlist = p->f.rowlist;
       fj.counts = p->f.counts;
-      cudaError_t e = cudaMemcpy(p->d_fft_tabs, tabs, sizeof(tabs), cudaMemcpyHostToDevice);
-      if (e == cudaSuccess) e = cudaMemcpy(p->d_mask_base, mb, sizeof(mb), cudaMemcpyHostToDevice);
-      if (e != cudaSuccess) st = cuda_status(e, "cudaMemcpy(fft tables)", __FILE__, __LINE__);
     }
   }
   // the sparse-aware path needs no cuFFT plan: the stage API creates it (and its
@@ -616,11 +610,9 @@ int rick_plan_destroy(rick_plan *p) {
   if (p->ing_copy) cudaStreamDestroy(p->ing_copy);
   for (cudaEvent_t e : p->ing_ev)
     if (e) cudaEventDestroy(e);
-  void *ptrs[] = {p->cube, p->s.bin_count, p->s.bin_cursor, p->s.item_off, p->s.scan_tmp,
-                  p->s.counters, p->s.records, p->s.table, p->d_lm, p->fft_work, p->h_rows_d,
-                  p->d_img, p->d_stage, p->d_norm, p->f.rowmask, p->f.rowbits, p->f.rowlist, p->f.counts,
-                  p->f.tw_x, p->f.tw_y, p->f.blocked,
-                  p->f.tilemask, p->d_job, p->d_fft_tabs, p->d_mask_base};
+  void *ptrs[] = {p->cube, p->d_clear, p->s.item_off, p->s.scan_tmp, p->s.records, p->s.table,
+                  p->d_lm, p->fft_work, p->h_rows_d, p->d_img, p->d_stage, p->d_norm, p->f.rowbits,
+                  p->f.rowlist, p->f.tw_x, p->f.tw_y, p->f.blocked};
   for (void *q : ptrs)
     if (q) cudaFree(q);
   if (p->h_lm) cudaFreeHost(p->h_lm);

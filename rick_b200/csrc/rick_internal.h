@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <cmath>
 
 #include "rick_b200.h"
 
@@ -54,18 +55,31 @@ struct Geometry {
   int half;             // KernelLen = (w_support-1)/2
   int ntx, nty;         // tiles per row / column
   double dx, dw;        // 1/Nx, 1/Nw (init.c:11-12) or as passed to wstack
+  double inv_dx, inv_dw; // 1/dx, 1/dw where those are powers of two, else 0 (set_spacing)
   double w_supporth;    // (double)half*dx (init.c:13)
   int select_sector0;   // apply gridding.c:149-188 membership
   int w_first;          // first plane of a w-plane shard (nw planes from here)
   int nw_total;         // planes of the whole cube (0: nw)
   uint64_t nbins() const { return (uint64_t)nw * ntx * nty; }
+  // Cell sizes.  A quotient by a power of two is the product with its inverse, to
+  // the bit, so the row passes skip the division there.
+  void set_spacing(double dx_, double dw_) {
+    auto inverse = [](double d) {
+      int e = 0;
+      return d > 0.0 && std::frexp(d, &e) == 0.5 && e > -1000 && e < 1000 ? 1.0 / d : 0.0;
+    };
+    dx = dx_;
+    dw = dw_;
+    inv_dx = inverse(dx_);
+    inv_dw = inverse(dw_);
+  }
 };
 
-// Binned row record (32 bytes: one DRAM sector, two 16-byte loads).  pu, pv
+// Binned row record (32 bytes: one DRAM sector, one 32-byte load or store).  pu, pv
 // are the FP64 pixel positions u/dx, v/dx of w-stacking.cu:143-144; the
 // gridder re-derives the cell (int)pos and the fraction pos - (int)pos, exact
 // in FP64, so (d + 0.5) - f rounds to the reference's (j + 0.5) - pos exactly.
-struct __align__(16) RecF64 {
+struct __align__(32) RecF64 {
   double sre, sim;   // sum over channels and polarisations of weight*vis
   double pu, pv;     // pixel position
 };
@@ -75,7 +89,7 @@ struct Scratch {
   uint32_t *bin_count = nullptr;   // [nbins+1] counts, then exclusive offsets
   uint32_t *bin_cursor = nullptr;  // [nbins]
   uint32_t *item_off = nullptr;    // [nbins+1] work-item offsets
-  uint32_t *scan_tmp = nullptr;    // block sums for the scans
+  uint32_t *scan_tmp = nullptr;    // block sums for the scan
   uint64_t *counters = nullptr;    // [8] device counters (see Counter)
   RecF64 *records = nullptr;       // [max_records]
   uint64_t max_records = 0;
@@ -104,7 +118,7 @@ struct BatchJob {
   uint64_t nrows;                  // rows of the job
   uint32_t nchan, npol;
   int scatter_lanes;               // lanes per row of the sample pass (1, 2, 4, ..., 32)
-  int scatter_v4;                  // 16-byte sample loads (aligned rows, nchan*npol % 4 == 0)
+  int scatter_vec;                 // samples per load of the sample pass (sample_vector)
   uint32_t bin_base;               // first global bin (nw*nty*ntx bins per job)
   uint32_t counts_base;            // first word of the job's [1 + nw] row counts
   uint64_t mask_base;              // first word of the job's row mask [nw * nty]
@@ -145,7 +159,6 @@ struct FftJobs {
   const uint32_t *col_units = nullptr;  // device [njobs + 1], in col_jobs order
   const uint64_t *mask_base = nullptr;  // device [njobs + 1], row-mask words per job
   uint64_t total_mask_words = 0;
-  uint32_t total_count_words = 0;
   uint32_t *rowmask = nullptr, *tilemask = nullptr, *rowlist = nullptr, *counts = nullptr;
   uint16_t *rowbits = nullptr;          // two entries per row-mask word
   int cols_parts = 1;                   // blocks a unit's planes are dealt to (one job)
@@ -176,13 +189,10 @@ enum Counter : int {
 void make_table(int kernel, int support, double *tab);
 
 // Pipeline stages (bin.cu, grid.cu, phase.cu).
-int bin_rows(const Geometry &g, int kernel, int precision, uint64_t nrows, const double *uu,
-             const double *vv, const double *ww, const float *weight, const float *vis_re,
-             const float *vis_im, uint32_t nchan, uint32_t npol, Scratch &s,
-             uint32_t max_chunk, cudaStream_t st, cudaEvent_t mid = nullptr);
-// The two passes of bin_rows, for callers that stream the samples in slices.
+// Both passes expect bin_count [nbins + 1] and bin_cursor [nbins] cleared.
 int bin_count_rows(const Geometry &g, uint64_t nrows, const double *uu, const double *vv,
                    const double *ww, Scratch &s, uint32_t max_chunk, cudaStream_t st);
+// The samples of all counted rows, or of successive slices of them.
 int bin_scatter_rows(const Geometry &g, uint64_t nrows, const double *uu, const double *vv,
                      const double *ww, const float *weight, const float *vis_re,
                      const float *vis_im, uint32_t nchan, uint32_t npol, Scratch &s,
@@ -208,8 +218,10 @@ int phase_sum(int precision, const void *cube, int xaxis, int yaxis, int nw, int
 // gridding.c:21-83 on device rows (uvw.cu); scratch: RICK_NORMALIZE_SCRATCH bytes.
 int normalize_uvw(uint64_t n, double *uu, double *vv, double *ww, void *scratch,
                   cudaStream_t st);
-int exclusive_scan_u32(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *tmp,
-                       cudaStream_t st);
+// counts[0..nbins) -> exclusive offsets in place (counts[nbins] the total) and
+// item_off[0..nbins]: exclusive offsets of ceil(count / max_chunk) (scan.cu).
+int scan_bins(uint32_t *counts, uint32_t *item_off, uint64_t nbins, uint32_t max_chunk,
+              uint32_t *tmp, cudaStream_t st);
 uint64_t scan_tmp_words(uint64_t n);
 
 #ifdef __CUDACC__
@@ -228,11 +240,10 @@ __device__ __forceinline__ int batch_job_of(const U *__restrict__ base, int njob
 #endif
 
 // Batch stages: every job of the batch in one launch per kernel.
-// Jobs of one sample-pass schedule (lanes per row, 16-byte loads): entries
+// Jobs of one sample-pass schedule (lanes per row, samples per load): entries
 // lo..hi-1 of the schedule-ordered job list.
 struct ScatterClass {
-  int lanes;
-  bool v4;
+  int lanes, vec;
   int lo, hi;
   uint64_t units;  // 32-row units of the class
 };
@@ -244,7 +255,7 @@ struct BatchLaunch {
   const uint32_t *sc_jobs;   // device [njobs]: jobs grouped by sample-pass schedule
   const uint64_t *sc_units;  // device [njobs + 1]: 32-row unit prefix in that order
   int n_sc;
-  ScatterClass sc[12];
+  ScatterClass sc[18];
   uint64_t total_row_units;
   uint32_t total_bins;
   int max_support;
@@ -278,8 +289,11 @@ void batch_destroy(rick_batch *b);
 uint64_t batch_bytes(const rick_job_desc *jobs, int njobs, int precision);
 bool batch_cached_tuning(int precision, rick_batch_tuning *t);
 
-// Lanes per row of the sample pass for rows of `per_row` loads (bin.cu).
-int lanes_per_row(uint64_t per_row);
+// Samples per load of the sample pass (4, 2 or 1) for rows of nv samples in npol
+// polarisations at these addresses, and the lanes per row for rows of `per_row`
+// loads (skips: a shard that skips most rows) (bin.cu).
+int sample_vector(const float *vis_re, const float *vis_im, uint64_t nv, uint32_t npol);
+int lanes_per_row(uint64_t per_row, bool skips = false);
 
 int num_sms();
 

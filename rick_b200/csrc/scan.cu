@@ -1,6 +1,9 @@
-// Exclusive prefix sum of 32-bit counts (bin offsets, work-item offsets).
-// Reduce-then-scan: each block scans 4096 entries and writes its total; the
-// totals are scanned recursively and added back.  In-place use is allowed.
+// Offsets of the bins and of the gridder's work items: exclusive prefix sums of the
+// record counts and of ceil(count / max_chunk), both at once.  One block for up to
+// 8191 bins; beyond, a first kernel sums blocks of 8192 bins and a second adds the
+// sums before its block (read by every block: 512 at 4M bins) to the
+// block's own scan.  The scans of one sum at a time this replaces took seven
+// launches for 8,192 bins.
 #include "rick_internal.h"
 
 namespace rick {
@@ -8,85 +11,112 @@ namespace rick {
 namespace {
 
 constexpr int kScanThreads = 1024;
-constexpr int kScanPerThread = 4;
+constexpr int kScanPerThread = 8;
 constexpr int kScanBlock = kScanThreads * kScanPerThread;
 
-__device__ __forceinline__ uint32_t warp_inclusive(uint32_t v) {
+// Records and work items, summed together.
+struct Sum2 {
+  uint32_t rec, items;
+};
+__device__ __forceinline__ Sum2 operator+(Sum2 a, Sum2 b) {
+  return {a.rec + b.rec, a.items + b.items};
+}
+
+__device__ __forceinline__ Sum2 warp_inclusive(Sum2 v) {
   const unsigned lane = threadIdx.x & 31u;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= (unsigned)o) v += t;
+    const Sum2 t = {__shfl_up_sync(0xffffffffu, v.rec, o), __shfl_up_sync(0xffffffffu, v.items, o)};
+    if (lane >= (unsigned)o) v = v + t;
   }
   return v;
 }
 
-// Scans one block of kScanBlock entries of `in` into `out` (exclusive) and
-// stores the block total in sums[blockIdx.x] (if sums != nullptr).
-__global__ void __launch_bounds__(kScanThreads)
-    k_scan_block(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *sums) {
-  __shared__ uint32_t warp_tot[kScanThreads / 32];
-  const uint64_t base = (uint64_t)blockIdx.x * kScanBlock + (uint64_t)threadIdx.x * kScanPerThread;
-  uint32_t v[kScanPerThread];
-  uint32_t local = 0;
-#pragma unroll
-  for (int k = 0; k < kScanPerThread; k++) {
-    v[k] = (base + k < n) ? in[base + k] : 0u;
-    local += v[k];
-  }
-  const uint32_t incl = warp_inclusive(local);
+// Exclusive prefix of each thread's value over the block, and the block's total.
+__device__ __forceinline__ Sum2 block_exclusive(Sum2 v, Sum2 &total) {
+  __shared__ Sum2 warp_tot[kScanThreads / 32];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const Sum2 incl = warp_inclusive(v);
+  __syncthreads();  // warp_tot of an earlier call is no longer read
   if (lane == 31) warp_tot[warp] = incl;
   __syncthreads();
-  if (warp == 0) {
-    uint32_t t = warp_tot[lane];
-    const uint32_t ti = warp_inclusive(t);
-    warp_tot[lane] = ti - t;  // exclusive over warps
-  }
-  __syncthreads();
-  uint32_t run = warp_tot[warp] + incl - local;
-#pragma unroll
-  for (int k = 0; k < kScanPerThread; k++) {
-    if (base + k < n) out[base + k] = run;
-    run += v[k];
-  }
-  if (sums && threadIdx.x == kScanThreads - 1) sums[blockIdx.x] = run;
+  const Sum2 t = warp_inclusive(warp_tot[lane]);  // every warp scans the warps' totals
+  total = {__shfl_sync(0xffffffffu, t.rec, 31), __shfl_sync(0xffffffffu, t.items, 31)};
+  const int src = warp == 0 ? 0 : (int)warp - 1;
+  const Sum2 before = {__shfl_sync(0xffffffffu, t.rec, src), __shfl_sync(0xffffffffu, t.items, src)};
+  const Sum2 own = {incl.rec - v.rec, incl.items - v.items};
+  return warp == 0 ? own : own + before;
 }
 
-__global__ void k_scan_add(uint32_t *out, uint64_t n, const uint32_t *sums) {
-  const uint32_t add = sums[blockIdx.x];
-  const uint64_t base = (uint64_t)blockIdx.x * kScanBlock;
-  for (int k = threadIdx.x; k < kScanBlock; k += blockDim.x)
-    if (base + k < n) out[base + k] += add;
+__device__ __forceinline__ Sum2 bin_sum(uint32_t c, uint32_t max_chunk) {
+  return {c, (c + max_chunk - 1) / max_chunk};
+}
+
+__global__ void __launch_bounds__(kScanThreads)
+    k_scan_sums(const uint32_t *__restrict__ counts, uint64_t nbins, uint32_t max_chunk,
+                Sum2 *__restrict__ sums) {
+  const uint64_t base = (uint64_t)blockIdx.x * kScanBlock + threadIdx.x;
+  Sum2 local = {0, 0}, total;
+#pragma unroll
+  for (int k = 0; k < kScanPerThread; k++) {
+    const uint64_t i = base + (uint64_t)k * kScanThreads;
+    if (i < nbins) local = local + bin_sum(counts[i], max_chunk);
+  }
+  block_exclusive(local, total);
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+// sums: the totals of the blocks (null for a single block).
+__global__ void __launch_bounds__(kScanThreads)
+    k_scan_bins(uint32_t *__restrict__ counts, uint32_t *__restrict__ item_off, uint64_t nbins,
+                uint32_t max_chunk, const Sum2 *__restrict__ sums) {
+  Sum2 before = {0, 0}, total;
+  if (sums) {
+    Sum2 part = {0, 0};
+    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += kScanThreads) part = part + sums[b];
+    block_exclusive(part, before);
+  }
+  const uint64_t base = (uint64_t)blockIdx.x * kScanBlock + (uint64_t)threadIdx.x * kScanPerThread;
+  Sum2 v[kScanPerThread], local = {0, 0};
+#pragma unroll
+  for (int k = 0; k < kScanPerThread; k++) {
+    v[k] = bin_sum(base + k < nbins ? counts[base + k] : 0u, max_chunk);
+    local = local + v[k];
+  }
+  Sum2 run = before + block_exclusive(local, total);
+#pragma unroll
+  for (int k = 0; k < kScanPerThread; k++) {
+    if (base + k <= nbins) {  // entry nbins: the totals
+      counts[base + k] = run.rec;
+      item_off[base + k] = run.items;
+    }
+    run = run + v[k];
+  }
 }
 
 }  // namespace
 
+// Two words a block of 8192 bins, with room to spare.
 uint64_t scan_tmp_words(uint64_t n) {
   uint64_t words = 0;
-  while (n > (uint64_t)kScanBlock) {
-    n = (n + kScanBlock - 1) / kScanBlock;
+  while (n > 4096) {
+    n = (n + 4095) / 4096;
     words += n;
   }
   return words + 64;
 }
 
-int exclusive_scan_u32(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *tmp,
-                       cudaStream_t st) {
-  if (n == 0) return RICK_OK;
-  if (n <= (uint64_t)kScanBlock) {
+int scan_bins(uint32_t *counts, uint32_t *item_off, uint64_t nbins, uint32_t max_chunk,
+              uint32_t *tmp, cudaStream_t st) {
+  const uint64_t nb = (nbins + 1 + kScanBlock - 1) / kScanBlock;
+  Sum2 *sums = nb > 1 ? (Sum2 *)tmp : nullptr;
+  if (sums) {
     RICK_LAUNCHED();
-    k_scan_block<<<1, kScanThreads, 0, st>>>(in, out, n, nullptr);
+    k_scan_sums<<<(unsigned)nb, kScanThreads, 0, st>>>(counts, nbins, max_chunk, sums);
     RICK_CUDA(cudaGetLastError());
-    return RICK_OK;
   }
-  const uint64_t nb = (n + kScanBlock - 1) / kScanBlock;
   RICK_LAUNCHED();
-  k_scan_block<<<(unsigned)nb, kScanThreads, 0, st>>>(in, out, n, tmp);
-  RICK_CUDA(cudaGetLastError());
-  RICK_TRY(exclusive_scan_u32(tmp, tmp, nb, tmp + nb, st));
-  RICK_LAUNCHED();
-  k_scan_add<<<(unsigned)nb, 256, 0, st>>>(out, n, tmp);
+  k_scan_bins<<<(unsigned)nb, kScanThreads, 0, st>>>(counts, item_off, nbins, max_chunk, sums);
   RICK_CUDA(cudaGetLastError());
   return RICK_OK;
 }
