@@ -373,8 +373,8 @@ __global__ void __launch_bounds__(Shape<L>::kThreads, row_min_blocks<L>())
 // packed FP32) issue 2,600 cycles of a sub-partition, load/store pipe ~3,600 of
 // the SM (two exchanges 2,048, a wavefront per touched row ~1,130, the image);
 // with 16 warps an SM the two overlap in part: 5,850 measured.  Against two
-// columns a block in radix-8 passes: 3.42 -> 2.64 ms FP64 and 2.55 -> 1.40 mixed
-// (4096^2 x 32), 10.5 -> 7.2 ms FP64 (8192^2, 16 planes of 64) and 10.9 -> 6.7
+// columns a block in radix-8 passes: 3.42 -> 2.60 ms FP64 and 2.55 -> 1.31 mixed
+// (4096^2 x 32), 10.5 -> 6.9 ms FP64 (8192^2, 16 planes of 64) and 10.9 -> 6.5
 // mixed (8192^2 x 32).  Warp w of a block reaches lanes 32 (w % 4) ..
 // +31 (its lane quarter); the warps of one quarter split its columns.
 
@@ -388,6 +388,20 @@ template <typename S, int L> struct ColState {
   using T = std::conditional_t<kWide, double, S>;
 };
 
+// From 1024-point columns on the column pass leaves the sums, unit by unit, in the
+// gridded cube, which the row pass has read, and k_fft_finish applies P and turns
+// them into image rows.  Written by the column pass itself the image rows of a unit
+// are pieces of 8 or 16 bytes, a whole 32-byte sector of traffic each, and its last
+// warps compute P with little else in flight.  Column pass and finish, both ways:
+// 0.49 -> 0.23 ms FP64 and 0.36 -> 0.14 mixed (4096^2, one plane), 2.88 -> 0.99 and
+// 2.38 -> 0.63 (8192^2, one plane), 1.40 -> 1.31 ms mixed (4096^2 x 32), 7.2 -> 6.9 FP64
+// (8192^2 x 16 of 64).  Clusters of blocks that write whole sectors together were
+// slower, 3.9 ms for the 2.64 of 4096^2 x 32: with TMEM in use one block of a cluster
+// launch fits an SM.  The sums keep their type; a unit's row takes 16 bytes, a plane
+// of the cube in either form.  (Wide sums do not fit; their short columns lie side by
+// side in a block, so that their pieces meet in L2.)
+template <int L> constexpr bool kFinish = L >= 10;
+
 // The per-job inputs of the column pass.
 template <typename S> struct ColJob {
   const typename Vec<S>::t *cube;  // row transforms by column units
@@ -400,6 +414,7 @@ template <typename S> struct ColJob {
   double wmin, dw, dwnorm, norm;
   int phase_on;
   double *img_re, *img_im;
+  typename Vec<S>::t *sums;        // [units][ny], L = 13: [units][half][ny / 2] (kFinish)
 };
 
 // Unit u of one job, column u or columns 2u, 2u + 1 (with L = 13, half `half` of
@@ -452,7 +467,7 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
   };
   int iw = prev_plane(hi);
   if (iw < lo) {  // no data at all
-    if (add) return;
+    if (add || kFinish<L>) return;
 #pragma unroll
     for (int q = 0; q < kVpt; q++)
       for (int c = 0; c < NL; c++) {
@@ -563,6 +578,19 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
     iw = nxt;
     nxt = nxt2;
     nbits = nbits2;
+  }
+  if constexpr (kFinish<L>) {
+    if (!add) {
+      V *to = J.sums + (uint64_t)u * ny + half * F::N + t;
+#pragma unroll 4
+      for (int q = 0; q < kVpt; q++) {
+        uint32_t a4[4];
+        tm::ld4(taddr + 4 * q, a4);
+        tm::wait_ld4(a4);
+        to[G * q] = fft::pack(Cx<S>{tm::join<S>(a4), tm::join<S>(a4 + 2)});
+      }
+      return;
+    }
   }
   // image = norm * P * sum, P the factor of the lowest plane with data
   const double cw = __dmul_rn(twopi, __dadd_rn(J.wmin, __dmul_rn((double)(J.w_first + prev), J.dw)));
@@ -721,11 +749,132 @@ __global__ void __launch_bounds__(Shape<L>::kThreads, col_blocks<S, L>())
       J.phase_on = B.phase_on;
       J.img_re = B.img_re;
       J.img_im = B.img_im;
+      J.sums = (V *)B.cube;
     }
     __syncthreads();
     fft_col_unit<S, L>(s, s_unit + grp, 0, 0, sJ.nw, false, t, sJ, tmem.addr);
   }
   tmem.release();
+}
+
+// image = norm * P * sum, P the factor of the lowest plane with data, from the sums
+// of a column pass with 2^L rows: 32 columns by 32 rows m below ny / 2 and their
+// mirror images ny - m (ny / 2 for m = 0) a block, read along the columns (512 bytes a
+// warp) and written along the rows.  FP64 sums and the image cross HBM once, 32 bytes
+// a pixel (0.083 ms at 4096^2); a sincos and a root a pixel take as long, so rows m
+// and ny - m, whose m^2 and with it P agree on a table of equal halves, share them
+// (523 -> 461 us for the 2048-row jobs of a mixed batch of 64).
+constexpr int kTile = 32;
+template <typename S> using FinishTile = typename Vec<S>::t[2][kTile / kLanes<S>][kTile + 1];
+template <typename S, int L>
+__device__ __forceinline__ void finish_tile(FinishTile<S> &tile, uint32_t n0, uint32_t m0, int low,
+                                            const ColJob<S> &J) {
+  constexpr int NL = kLanes<S>;
+  const uint32_t lane = threadIdx.x % 32, warp = threadIdx.x / 32, warps = blockDim.x / 32;
+  const uint32_t ny = (uint32_t)J.ny;
+  auto mirror = [&](uint32_t m) { return m ? ny - m : ny / 2; };
+  if (low < J.nw) {
+    auto at = [](uint32_t m) { return Shape<L>::kSplit ? m % 2 * Shape<L>::N + m / 2 : m; };
+    const uint32_t at0 = at(m0 + lane), at1 = at(mirror(m0 + lane));
+#pragma unroll 4
+    for (uint32_t i = warp; i < kTile / NL; i += warps) {
+      const typename Vec<S>::t *from = J.sums + (uint64_t)(n0 / NL + i) * ny;
+      tile[0][i][lane] = __ldcs(from + at0);
+      tile[1][i][lane] = __ldcs(from + at1);
+    }
+  }
+  __syncthreads();
+  const bool phase = J.phase_on && J.nw_total > 1;
+  const double cw = __dmul_rn(2.0 * kPi, __dadd_rn(J.wmin, __dmul_rn((double)(J.w_first + low), J.dw)));
+  const double l = J.ltab[n0 + lane], l2 = __dmul_rn(l, l);
+#pragma unroll 1
+  for (uint32_t i = warp; i < kTile; i += warps) {
+    double mm = -1.0, pr = 1.0, pi = 0.0;
+#pragma unroll 1
+    for (int h = 0; h < 2; h++) {
+      const uint32_t m = h ? mirror(m0 + i) : m0 + i;
+      double re = 0.0, im = 0.0;
+      if (low < J.nw) {
+        const double m2 = __dmul_rn(J.mtab[m], J.mtab[m]);
+        if (phase && m2 != mm) {
+          const double root = __dsqrt_rn(__dsub_rn(1.0, __dadd_rn(l2, m2)));
+          double sn, cs;
+          sincos(__dmul_rn(cw, __dsub_rn(root, 1.0)), &sn, &cs);
+          const double amp = J.dwnorm * root;
+          pr = cs * amp;
+          pi = sn * amp;
+          mm = m2;
+        }
+        const Cx<S> x = fft::unpack(tile[h][lane / NL][i]);
+        double ar, ai;
+        if constexpr (NL == 2) {
+          ar = lane % 2 ? x.re.y : x.re.x;
+          ai = lane % 2 ? x.im.y : x.im.x;
+        } else {
+          ar = x.re;
+          ai = x.im;
+        }
+        re = J.norm * fma(ar, pr, -ai * pi);
+        im = J.norm * fma(ar, pi, ai * pr);
+      }
+      const uint64_t o = (uint64_t)m * (uint32_t)J.nx + n0 + lane;
+      __stcs(J.img_re + o, re);
+      __stcs(J.img_im + o, im);
+    }
+  }
+}
+
+// The lowest of a job's planes with data (nw: none), by a whole warp.
+__device__ __forceinline__ int lowest_plane(const uint32_t *counts, int nw) {
+  for (int w = 0; w < nw; w += 32) {
+    const int k = w + (int)(threadIdx.x % 32);
+    const uint32_t have = __ballot_sync(0xffffffffu, k < nw && __ldg(counts + 1 + k) > 0);
+    if (have) return w + __ffs(have) - 1;
+  }
+  return nw;
+}
+
+constexpr int kFinishThreads = 256;
+
+template <typename S, int L>
+__global__ void __launch_bounds__(kFinishThreads) k_fft_finish(ColJob<S> J) {
+  __shared__ FinishTile<S> tile;
+  const uint32_t across = (uint32_t)J.nx / kTile;
+  const int low = lowest_plane(J.counts, J.nw);
+  finish_tile<S, L>(tile, blockIdx.x % across * kTile, blockIdx.x / across * kTile, low, J);
+}
+
+// Of the jobs col_jobs[lo..hi-1] of a batch: a block's worth of units holds
+// `per_block` tiles.
+template <typename S, int L>
+__global__ void __launch_bounds__(kFinishThreads)
+    k_fft_finish_multi(const BatchJob *__restrict__ jobs, const uint32_t *__restrict__ col_jobs, int lo,
+                       int hi, const uint32_t *__restrict__ col_units, const uint32_t *__restrict__ counts) {
+  constexpr uint32_t per_block = kLanes<S> * Shape<L>::kGroups * (1u << L) / (2 * kTile * kTile);
+  __shared__ FinishTile<S> tile;
+  const uint32_t b = col_units[lo] + blockIdx.x / per_block;
+  const int k = lo + batch_job_of(col_units + lo, hi - lo, b);
+  const BatchJob &B = jobs[col_jobs[k]];
+  ColJob<S> J;
+  J.nx = B.g.nx;
+  J.ny = B.g.ny;
+  J.nw = B.g.nw;
+  J.w_first = B.g.w_first;
+  J.nw_total = B.g.nw_total > 0 ? B.g.nw_total : B.g.nw;
+  J.ltab = B.ltab;
+  J.mtab = B.mtab;
+  J.wmin = B.wmin;
+  J.dw = B.dw_phase;
+  J.dwnorm = B.dwnorm;
+  J.norm = B.norm;
+  J.phase_on = B.phase_on;
+  J.img_re = B.img_re;
+  J.img_im = B.img_im;
+  J.sums = (typename Vec<S>::t *)B.cube;
+  const uint32_t i = blockIdx.x - (col_units[k] - col_units[lo]) * per_block;
+  const uint32_t across = (uint32_t)J.nx / kTile;
+  finish_tile<S, L>(tile, i % across * kTile, i / across * kTile,
+                    lowest_plane(counts + B.counts_base, J.nw), J);
 }
 
 // ---- Lists -------------------------------------------------------------------------
@@ -780,18 +929,27 @@ __global__ void k_row_list(const BatchJob *__restrict__ jobs, const __grid_const
 }
 
 // Row-pass units per job (blocks' worths of touched rows of its x length, `lanes`
-// rows to a group), exclusive prefix over the jobs; one thread (a few hundred
-// jobs at most).
+// rows to a group), exclusive prefix over the jobs, by one warp (one thread took
+// 26 us for 64 jobs; 4.5).
 __global__ void k_fft_units(const BatchJob *__restrict__ jobs, int njobs, int lanes,
                             const uint32_t *__restrict__ counts, uint32_t *__restrict__ fft_units) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
   uint32_t acc = 0;
-  for (int j = 0; j < njobs; j++) {
-    fft_units[j] = acc;
-    const uint32_t rpb = (uint32_t)(fft_groups_per_block(jobs[j].logx) * lanes);
-    acc += (counts[jobs[j].counts_base] + rpb - 1) / rpb;
+  for (int j0 = 0; j0 < njobs; j0 += 32) {
+    const int j = j0 + (int)threadIdx.x;
+    uint32_t n = 0;
+    if (j < njobs) {
+      const uint32_t rpb = (uint32_t)(fft_groups_per_block(jobs[j].logx) * lanes);
+      n = (counts[jobs[j].counts_base] + rpb - 1) / rpb;
+    }
+    uint32_t upto = n;  // inclusive over the warp
+    for (int d = 1; d < 32; d *= 2) {
+      const uint32_t below = __shfl_up_sync(0xffffffffu, upto, d);
+      if ((int)threadIdx.x >= d) upto += below;
+    }
+    if (j < njobs) fft_units[j] = acc + upto - n;
+    acc += __shfl_sync(0xffffffffu, upto, 31);
   }
-  fft_units[njobs] = acc;
+  if (threadIdx.x == 0) fft_units[njobs] = acc;
 }
 
 // Longest transform of the multi-job (batch) kernels: 4096.
@@ -817,6 +975,7 @@ template <typename S> ColJob<S> col_job(const BatchJob &B, const FftJobs &f) {
   J.phase_on = B.phase_on;
   J.img_re = B.img_re;
   J.img_im = B.img_im;
+  J.sums = (typename Vec<S>::t *)B.cube;
   return J;
 }
 
@@ -886,11 +1045,25 @@ int launch_cols(const FftJobs &f, const FftClass &c, cudaStream_t st) {
     const uint64_t nb = (uint64_t)B.g.nx / kLanes<S> / F::kGroups * (F::kSplit ? 2 : 1);
     const int parts = f.cols_parts;
     const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(nb * parts, slots));
-    k_fft_cols<S, L><<<blocks, BT, sm, st>>>(col_job<S>(B, f), parts);
+    const ColJob<S> J = col_job<S>(B, f);
+    k_fft_cols<S, L><<<blocks, BT, sm, st>>>(J, parts);
+    if constexpr (kFinish<L>) {
+      if (parts == 1) {
+        RICK_LAUNCHED();
+        const uint64_t tiles = (uint64_t)J.nx * J.ny / (2 * kTile * kTile);
+        k_fft_finish<S, L><<<(unsigned)tiles, kFinishThreads, 0, st>>>(J);
+      }
+    }
   } else if constexpr (L <= kMultiMaxLog) {
     const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(c.units, slots));
     k_fft_cols_multi<S, L><<<blocks, BT, sm, st>>>(f.jobs, f.col_jobs, c.lo, c.hi, f.col_units,
                                                    f.rowbits, f.counts);
+    if constexpr (kFinish<L>) {
+      RICK_LAUNCHED();
+      const uint64_t tiles = c.units * (uint64_t)(kLanes<S> * F::kGroups * (1 << L) / (2 * kTile * kTile));
+      k_fft_finish_multi<S, L><<<(unsigned)tiles, kFinishThreads, 0, st>>>(
+          f.jobs, f.col_jobs, c.lo, c.hi, f.col_units, f.counts);
+    }
   }
   RICK_CUDA(cudaGetLastError());
   return RICK_OK;
