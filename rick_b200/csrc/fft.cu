@@ -163,8 +163,8 @@ template <> __device__ __forceinline__ float2 join<float2>(const uint32_t *w) {
 // odd outputs in the two lanes, which are the two columns of a unit -- mixed.
 // Bound by the write of the transformed rows (36,060 rows of 4096: 2.4 GB FP64)
 // and, below that, by the load/store pipe: the exchanges and the sector-wide
-// stores.  Measured at 4096^2 x 32 / 8192^2: 0.96 / 2.7 ms FP64 (0.93 / 2.7 with
-// radix-8 passes and line-wide stores), 0.49 / 1.6 ms mixed (0.63 / 2.1).
+// stores.  Measured at 4096^2 x 32 / 8192^2: 0.90 / 2.2 ms FP64 (0.93 / 2.7 with
+// radix-8 passes and line-wide stores), 0.45 / 1.5 ms mixed (0.63 / 2.1).
 template <typename S, int L> struct RowShape {
   using F = Shape<L>;
   static constexpr bool kBothHalves = F::kSplit && kLanes<S> == 2;
@@ -173,52 +173,72 @@ template <typename S, int L> struct RowShape {
 };
 
 struct RowSrc {
-  const uint32_t *tm;  // the row's tile bitmap words
-  uint64_t base;       // its first element in the cube
+  uint64_t base;  // the row's first element in the cube
+  uint32_t bits;  // bit r: the tile of the thread's input r (x = t + G r) has records
   uint32_t w, k;
   bool active;
 };
 
-// Input r (x = t + G r) of the group's rows.
+// Input r (x = t + G r) of the group's rows, as the first loads leave it; row_inputs
+// makes the inputs of these.  At 8192 points that takes a second cell (x + N): FP64
+// rows read it there (2.74 -> 2.23 ms for 8192^2, 16 planes of 64), the mixed form
+// reads both there (1.54 ms for 8192^2 x 32, 1.58 with its cells read early: spills).
 template <typename S, int L>
-__device__ __forceinline__ Cx<S> row_input(const RowSrc (&src)[kLanes<S>], int half, int t, int r,
+__device__ __forceinline__ Cx<S> row_input(const RowSrc (&src)[kLanes<S>], int t, int r,
                                            const typename CubeVec<S>::t *__restrict__ cube) {
   using F = Shape<L>;
-  using C = typename CubeVec<S>::t;
-  auto cell = [&](const RowSrc &q, int x) {
-    C v;
+  auto cell = [&](const RowSrc &q, int r) {
+    typename CubeVec<S>::t v;
     v.x = 0;
     v.y = 0;
-    if (q.active && ((__ldg(q.tm + (x >> 10)) >> ((x >> 5) & 31)) & 1u)) v = __ldg(cube + q.base + x);
+    if ((q.bits >> r) & 1u) v = __ldg(cube + q.base + t + F::G * r);
     return v;
   };
-  const int x = t + F::G * r;
-  const C a = cell(src[0], x);
-  if constexpr (F::kSplit) {
-    const C b = cell(src[0], x + F::N);
-    if constexpr (kLanes<S> == 2)
-      return {make_float2(a.x + b.x, a.x - b.x), make_float2(a.y + b.y, a.y - b.y)};
-    else
-      return half ? Cx<S>{a.x - b.x, a.y - b.y} : Cx<S>{a.x + b.x, a.y + b.y};
-  } else if constexpr (kLanes<S> == 2) {
-    const C b = cell(src[1], x);
+  const auto a = cell(src[0], r);
+  if constexpr (kLanes<S> == 2) {
+    const auto b = F::kSplit ? cell(src[0], 16 + r) : cell(src[1], r);
     return {make_float2(a.x, b.x), make_float2(a.y, b.y)};
   } else {
     return {a.x, a.y};
   }
 }
-
-// The rows whose inputs v holds: transformed and written.
 template <typename S, int L>
+__device__ __forceinline__ void row_inputs(const RowSrc (&src)[kLanes<S>], int half, int t,
+                                           const typename CubeVec<S>::t *__restrict__ cube,
+                                           Cx<S> (&v)[kVpt]) {
+  if constexpr (RowShape<S, L>::kBothHalves) {
+#pragma unroll
+    for (int r = 0; r < kVpt; r++) v[r] = row_input<S, L>(src, t, r, cube);
+  }
+  if constexpr (Shape<L>::kSplit) {
+#pragma unroll
+    for (int r = 0; r < kVpt; r++) {
+      if constexpr (kLanes<S> == 2) {
+        v[r] = {make_float2(v[r].re.x + v[r].re.y, v[r].re.x - v[r].re.y),
+                make_float2(v[r].im.x + v[r].im.y, v[r].im.x - v[r].im.y)};
+      } else {
+        Cx<S> b = {0.0, 0.0};
+        if ((src[0].bits >> (16 + r)) & 1u)
+          b = fft::unpack(__ldg(cube + src[0].base + t + Shape<L>::G * r + Shape<L>::N));
+        v[r] = half ? Cx<S>{v[r].re - b.re, v[r].im - b.im} : Cx<S>{v[r].re + b.re, v[r].im + b.im};
+      }
+    }
+  }
+}
+
+// The rows whose inputs v holds: transformed and written.  mid() runs between the
+// passes, next(q) when v[q] is written.
+template <typename S, int L, typename Mid, typename Next>
 __device__ __forceinline__ void fft_row_unit(typename Vec<S>::t *s, const RowSrc (&src)[kLanes<S>],
                                              int half, int t,
                                              typename Vec<S>::t *__restrict__ out, int nx, int ny,
                                              const typename fft::TwVec<S>::t *__restrict__ tw,
-                                             Cx<S> (&v)[kVpt]) {
+                                             Cx<S> (&v)[kVpt], Mid mid, Next next) {
   using F = Shape<L>;
   using RS = RowShape<S, L>;
   constexpr int G = F::G;
   fft::first_pass<L, S>(s, t, RS::kBothHalves ? fft::kBoth : half, v);
+  mid();
   if constexpr (RS::kBothHalves) {
     fft::later_passes<L, S>(s, t, [&](int e) { return fft::twiddle(tw + e, tw + F::kTab + e); }, v);
   } else {
@@ -229,13 +249,17 @@ __device__ __forceinline__ void fft_row_unit(typename Vec<S>::t *s, const RowSrc
     const uint32_t u0 = F::kSplit ? half * F::N + t : t;  // unit_of
     auto *o = out + unit_base(src[0].w, u0, nx, ny) + (uint64_t)src[0].k * kUnitBlock;
 #pragma unroll
-    for (int q = 0; q < kVpt; q++)
+    for (int q = 0; q < kVpt; q++) {
       if (src[0].active) o[(uint64_t)(G * q) * ny] = fft::pack(v[q]);
+      next(q);
+    }
   } else if constexpr (RS::kBothHalves) {
     auto *o = out + unit_base(src[0].w, t, nx / 2, ny) + (uint64_t)src[0].k * kUnitBlock;
 #pragma unroll
-    for (int q = 0; q < kVpt; q++)
+    for (int q = 0; q < kVpt; q++) {
       if (src[0].active) o[(uint64_t)(G * q) * ny] = fft::pack(v[q]);
+      next(q);
+    }
   } else {
     // columns n, n + 1 are neighbouring lanes' outputs: the even lane takes
     // both for the first row, the odd lane for the second
@@ -252,24 +276,41 @@ __device__ __forceinline__ void fft_row_unit(typename Vec<S>::t *s, const RowSrc
         // pair-units of a G-aligned step: G/2 units, in blocks of kUnitBlock
         o[(uint64_t)(G / 2 * q) * ny] = fft::pack(c);
       }
+      next(q);
     }
   }
 }
 
-// Row list entries li, li + 1, ... of a group (a job's arrays).
+// Row list entries li, li + 1, ... of a group (a job's arrays): their ids (all bits
+// set past the list's end), and the rows these stand for.
 template <typename S, int L>
-__device__ __forceinline__ void row_sources(RowSrc (&src)[kLanes<S>], uint32_t li, uint32_t nrows,
-                                            const uint32_t *__restrict__ rowlist, int nx, int ny,
-                                            int nty, int tmw, const uint32_t *__restrict__ tilemask) {
+__device__ __forceinline__ void row_ids(uint32_t (&id)[kLanes<S>], uint32_t li, uint32_t nrows,
+                                        const uint32_t *__restrict__ rowlist) {
+#pragma unroll
+  for (int i = 0; i < kLanes<S>; i++)
+    id[i] = i < RowShape<S, L>::kRows && li + i < nrows ? __ldg(rowlist + li + i) : ~0u;
+}
+template <typename S, int L>
+__device__ __forceinline__ void row_sources(RowSrc (&src)[kLanes<S>], const uint32_t (&id)[kLanes<S>],
+                                            int t, int nx, int ny, int nty, int tmw,
+                                            const uint32_t *__restrict__ tilemask) {
+  using F = Shape<L>;
 #pragma unroll
   for (int i = 0; i < kLanes<S>; i++) {
     RowSrc &r = src[i];
-    r.active = i < RowShape<S, L>::kRows && li + i < nrows;
-    const uint32_t rid = r.active ? rowlist[li + i] : 0;
+    r.active = id[i] != ~0u;
+    const uint32_t rid = r.active ? id[i] : 0;
     r.w = rid / (uint32_t)ny;
     r.k = rid % (uint32_t)ny;
-    r.tm = tilemask + ((uint64_t)r.w * nty + (r.k >> 5)) * tmw;
     r.base = ((uint64_t)r.w * ny + r.k) * nx;
+    r.bits = 0;
+    if (r.active) {
+      const uint32_t *tm = tilemask + ((uint64_t)r.w * nty + (r.k >> 5)) * tmw;
+      // input r is in tile (t + G r) / 32, a bit of word G r / 1024 (G divides 1024, t < G)
+#pragma unroll
+      for (int q = 0; q < (F::kSplit ? 32 : 16); q++)
+        r.bits |= ((__ldg(tm + (F::G * q >> 10)) >> (((t + F::G * q) >> 5) & 31)) & 1u) << q;
+    }
   }
 }
 
@@ -296,20 +337,36 @@ __global__ void __launch_bounds__(Shape<L>::kThreads, row_min_blocks<L>())
   auto *s = reinterpret_cast<typename Vec<S>::t *>(smem_raw) + grp * F::N;
   const uint32_t nrows = counts[0];
   const uint32_t units = (nrows + rows_per_block<S, L>() - 1) / rows_per_block<S, L>() * RS::kParts;
+  // a unit's row ids are read during the unit before it and their tile bits between
+  // its passes, so that of the three dependent reads only the cells' remains, and
+  // those start as the unit's values are written, each into the registers it frees
+  // (0.96 -> 0.90 ms FP64, 0.49 -> 0.45 mixed for 36,060 rows of 4096)
   Cx<S> v[kVpt];
-  RowSrc src[kLanes<S>];
-  auto load = [&](uint32_t u) {
-    row_sources<S, L>(src, u < units ? (u / RS::kParts * F::kGroups + grp) * RS::kRows : nrows, nrows,
-                      rowlist, nx, ny, nty, tmw, tilemask);
-#pragma unroll
-    for (int r = 0; r < kVpt; r++)
-      v[r] = row_input<S, L>(src, RS::kParts == 2 ? (int)(u & 1) : 0, t, r, cube);
+  RowSrc src[kLanes<S>], nsrc[kLanes<S>];
+  uint32_t id[kLanes<S>];
+  auto ids = [&](uint32_t u) {
+    row_ids<S, L>(id, u < units ? (u / RS::kParts * F::kGroups + grp) * RS::kRows : nrows, nrows,
+                  rowlist);
   };
-  load(blockIdx.x);
+  auto half_of = [](uint32_t u) { return RS::kParts == 2 ? (int)(u & 1) : 0; };
+  ids(blockIdx.x);
+  row_sources<S, L>(src, id, t, nx, ny, nty, tmw, tilemask);
+#pragma unroll
+  for (int r = 0; r < kVpt; r++)
+    if (!RS::kBothHalves) v[r] = row_input<S, L>(src, t, r, cube);
   for (uint32_t u = blockIdx.x; u < units;) {
-    fft_row_unit<S, L>(s, src, RS::kParts == 2 ? (int)(u & 1) : 0, t, out, nx, ny, tw, v);
-    u += gridDim.x;
-    load(u);
+    const uint32_t un = u + gridDim.x;
+    row_inputs<S, L>(src, half_of(u), t, cube, v);
+    ids(un);
+    fft_row_unit<S, L>(
+        s, src, half_of(u), t, out, nx, ny, tw, v,
+        [&] { row_sources<S, L>(nsrc, id, t, nx, ny, nty, tmw, tilemask); },
+        [&](int q) {
+          if (!RS::kBothHalves) v[q] = row_input<S, L>(nsrc, t, q, cube);
+        });
+#pragma unroll
+    for (int i = 0; i < kLanes<S>; i++) src[i] = nsrc[i];
+    u = un;
   }
 }
 
@@ -331,16 +388,19 @@ __global__ void __launch_bounds__(Shape<L>::kThreads, row_min_blocks<L>())
   for (uint32_t u = fft_units[lo] + blockIdx.x; u < u1; u += gridDim.x) {
     const int j = lo + batch_job_of(fft_units + lo, hi - lo, u);
     const BatchJob &J = jobs[j];
+    uint32_t id[kLanes<S>];
     RowSrc src[kLanes<S>];
-    row_sources<S, L>(src, ((u - fft_units[j]) * F::kGroups + grp) * RS::kRows,
-                      counts[J.counts_base], rowlist + J.list_base, J.g.nx, J.g.ny, J.g.nty,
-                      (J.g.ntx + 31) / 32, tilemask + J.tile_base);
+    row_ids<S, L>(id, ((u - fft_units[j]) * F::kGroups + grp) * RS::kRows, counts[J.counts_base],
+                  rowlist + J.list_base);
+    row_sources<S, L>(src, id, t, J.g.nx, J.g.ny, J.g.nty, (J.g.ntx + 31) / 32,
+                      tilemask + J.tile_base);
     Cx<S> v[kVpt];
 #pragma unroll
     for (int r = 0; r < kVpt; r++)
-      v[r] = row_input<S, L>(src, 0, t, r, (const typename CubeVec<S>::t *)J.cube);
+      if (!RS::kBothHalves) v[r] = row_input<S, L>(src, t, r, (const typename CubeVec<S>::t *)J.cube);
+    row_inputs<S, L>(src, 0, t, (const typename CubeVec<S>::t *)J.cube, v);
     fft_row_unit<S, L>(s, src, 0, t, (V *)J.blocked, J.g.nx, J.g.ny,
-                       (const typename fft::TwVec<S>::t *)J.tw_x, v);
+                       (const typename fft::TwVec<S>::t *)J.tw_x, v, [] {}, [](int) {});
   }
 }
 
@@ -374,7 +434,7 @@ __global__ void __launch_bounds__(Shape<L>::kThreads, row_min_blocks<L>())
 // the SM (two exchanges 2,048, a wavefront per touched row ~1,130, the image);
 // with 16 warps an SM the two overlap in part: 5,850 measured.  Against two
 // columns a block in radix-8 passes: 3.42 -> 2.60 ms FP64 and 2.55 -> 1.31 mixed
-// (4096^2 x 32), 10.5 -> 6.9 ms FP64 (8192^2, 16 planes of 64) and 10.9 -> 6.5
+// (4096^2 x 32), 10.5 -> 6.9 ms FP64 (8192^2, 16 planes of 64) and 10.9 -> 6.3
 // mixed (8192^2 x 32).  Warp w of a block reaches lanes 32 (w % 4) ..
 // +31 (its lane quarter); the warps of one quarter split its columns.
 
@@ -563,14 +623,17 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
         }
         tm::split(fft::fma_(ar, sr, fft::fma_(fft::neg(ai), si, x.re)), sum + 4 * h);
         tm::split(fft::fma_(ar, si, fft::fma_(ai, sr, x.im)), sum + 4 * h + 2);
-        if constexpr (!F::kSplit)
+        if constexpr (!F::kSplit || NL == 2)
           if (M == 1 || h == 1) v[q] = row(col, nbits, q);
       }
       tm::st8(taddr + 4 * i0, sum);
     }
     if constexpr (F::kSplit) {
 #pragma unroll
-      for (int q = 0; q < kVpt; q++) v[q] = combine(row(col, nbits, q), row(col, nbits, 16 + q));
+      for (int q = 0; q < kVpt; q++) {  // (FP64 spills with the first rows read earlier)
+        if constexpr (NL == 1) v[q] = row(col, nbits, q);
+        v[q] = combine(v[q], row(col, nbits, 16 + q));
+      }
     }
     tm::wait_st();
     prev = iw;
