@@ -349,10 +349,10 @@ __device__ __forceinline__ void scatter_rows(
   const unsigned lane = lane_id();
   const unsigned sub = lane % G, grp = lane / G;
   const uint64_t nv = (uint64_t)nchan * npol;
-  // A w-plane shard (SHARD) holds a fraction of the rows: its rows of other
-  // planes (and rows that reach no tile) are found before any sample is read,
-  // so they never stream their samples.  A whole-cube plan keeps nearly every
-  // row and compiles without the check.
+  // With SHARD the rows of planes outside a w-plane shard (and rows that reach no
+  // tile) are found before any sample is read, so they never stream their samples
+  // (shard_schedule).  A whole-cube plan keeps nearly every row and compiles
+  // without the check.
   bool need = true;
   if (SHARD) {
     const uint64_t i_own = base + lane;
@@ -700,15 +700,41 @@ int bin_count_rows(const Geometry &g, uint64_t nrows, const double *uu, const do
 
 // Lanes that share one row's samples: one for rows of fewer than eight loads (a row
 // spread over lanes would leave each lane a load or two and the warp waiting), four
-// up to fifteen, then enough to cover the row's loads in one or two sweeps.  A shard
-// that holds less than half of the planes reads rows of eight loads a lane a row: it
-// skips rows one by one (2.8M of 3.8M rows: 0.32 ms against 0.35 with four lanes).
-int lanes_per_row(uint64_t per_row, bool skips) {
-  if (per_row < 8 || (skips && per_row == 8)) return 1;
-  if (per_row < 16) return skips ? 8 : 4;
-  int G = 16;
-  while (G < 32 && (uint64_t)G * 2 <= per_row) G *= 2;
-  return G;
+// up to fifteen, then enough to cover the row's loads in one or two sweeps.
+int lanes_per_row(uint64_t per_row) {
+  if (per_row < 8) return 1;
+  if (per_row < 16) return 4;
+  return per_row < 32 ? 16 : 32;
+}
+
+// The same for a w-plane shard, and whether its rows of other planes are found
+// before any sample is read (`skip`).  A whole-cube plan's schedules read every row;
+// a shard leaves them where skipping is faster, on 1.5M rows with their planes in
+// random order / in runs of 64 rows (us, the shard keeping half of the rows):
+//   * 32 loads and more: 32 lanes, skipping (64 loads: 341 / 416 against 524 / 520
+//     reading every row, 500 / 510 against 532 / 528 with nine tenths kept);
+//   * 16 to 31: eight lanes, skipping (24 loads: 271 / 232 against 404 / 399 reading
+//     every row and 408 / 387 skipping with sixteen lanes; 309 / 301 against 410 /
+//     407 and 496 / 487 with nine tenths kept);
+//   * 8 to 15: four lanes reading every row where the shard has half of the planes or
+//     more (12 loads: 150 / 144 against 268 / 222 skipping with eight lanes); below
+//     that up to 12 loads a lane a row with block-wise places, which skips (12 loads,
+//     a quarter of the rows kept: 111 / 103 against 222 / 164), and eight lanes beyond
+//     (15 loads, a third of the planes with 0.95 of the rows: 304 against 333);
+//   * fewer: block-wise places from half of the planes on, else a lane a row with
+//     places taken by warp (4 loads, a quarter kept: 76 / 56 against 74 / 61; all but
+//     a tenth: 106 / 90 against 115 / 102, but 176 against 115 on tracks, whose dense
+//     bins the block-wise places are for).
+struct SampleSchedule {
+  int lanes;
+  bool skip;  // one lane without skip: block-wise places (k_bin_scatter_short)
+};
+static SampleSchedule shard_schedule(uint64_t per_row, bool under_half) {
+  if (per_row >= 32) return {32, true};
+  if (per_row >= 16) return {8, true};
+  if (per_row >= 13 && under_half) return {8, true};
+  if (per_row >= 8) return {under_half ? 1 : 4, false};
+  return {1, under_half};
 }
 
 // 16-byte loads where the rows start on 16 bytes and a load's polarisations repeat
@@ -731,10 +757,12 @@ int bin_scatter_rows(const Geometry &g, uint64_t nrows, const double *uu, const 
   const uint64_t nv = (uint64_t)nchan * npol;
   const int N = sample_vector(vis_re, vis_im, nv, npol);
   const int sms = num_sms();
-  const bool skips = g.nw_total > 0 && 2 * g.nw < g.nw_total;
-  const int G = lanes_per_row(nv / N, skips);
+  const uint64_t per_row = nv / N;
+  SampleSchedule sch{lanes_per_row(per_row), false};
+  if (g.nw_total > 0 && g.nw != g.nw_total) sch = shard_schedule(per_row, 2 * g.nw < g.nw_total);
+  const int G = sch.lanes;
   RICK_LAUNCHED();
-  if (G == 1 && !skips) {
+  if (G == 1 && !sch.skip) {
     const uint64_t need = (nrows + kShortThreads - 1) / kShortThreads;
     const int blocks = (int)std::min<uint64_t>(need, (uint64_t)sms * 2);
 #define RICK_SHORT(NN)                                                                          \
@@ -748,19 +776,16 @@ int bin_scatter_rows(const Geometry &g, uint64_t nrows, const double *uu, const 
     return RICK_OK;
   }
   const int blocks = (int)std::min<uint64_t>(((nrows + 31) / 32 + 7) / 8, (uint64_t)sms * 8);
-#define RICK_LONG(GG, NN)                                                                        \
-  if (G == GG && N == NN) {                                                                      \
-    if (skips)                                                                                   \
-      k_bin_scatter<GG, NN, true><<<blocks, 256, 0, st>>>(uu, vv, ww, weight, vis_re, vis_im,    \
-                                                          nrows, nchan, npol, g, s.bin_count,    \
-                                                          s.bin_cursor, s.records, s.counters);  \
-    else                                                                                         \
-      k_bin_scatter<GG, NN, false><<<blocks, 256, 0, st>>>(uu, vv, ww, weight, vis_re, vis_im,   \
-                                                           nrows, nchan, npol, g, s.bin_count,   \
-                                                           s.bin_cursor, s.records, s.counters); \
-  }
-#define RICK_LANES(X, NN) X(1, NN) X(4, NN) X(8, NN) X(16, NN) X(32, NN)
-  RICK_LANES(RICK_LONG, 4) RICK_LANES(RICK_LONG, 2) RICK_LANES(RICK_LONG, 1)
+#define RICK_LONG(GG, NN, SKIP)                                                                  \
+  if (G == GG && N == NN && sch.skip == SKIP)                                                    \
+    k_bin_scatter<GG, NN, SKIP><<<blocks, 256, 0, st>>>(uu, vv, ww, weight, vis_re, vis_im,      \
+                                                        nrows, nchan, npol, g, s.bin_count,      \
+                                                        s.bin_cursor, s.records, s.counters);
+#define RICK_SCHEDULES(NN)                                                             \
+  RICK_LONG(4, NN, false) RICK_LONG(16, NN, false) RICK_LONG(32, NN, false)            \
+  RICK_LONG(1, NN, true) RICK_LONG(8, NN, true) RICK_LONG(32, NN, true)
+  RICK_SCHEDULES(4) RICK_SCHEDULES(2) RICK_SCHEDULES(1)
+#undef RICK_SCHEDULES
 #undef RICK_LONG
   RICK_CUDA(cudaGetLastError());
   return RICK_OK;
@@ -788,7 +813,9 @@ int bin_rows_batch(const BatchLaunch &b, Scratch &s, uint32_t max_chunk, cudaStr
     k_bin_scatter_batch<GG, NN><<<blocks, 256, 0, st>>>(b.jobs, b.sc_jobs, b.sc_units, k.lo, \
                                                         k.hi, s.bin_count, s.bin_cursor,     \
                                                         s.records, s.counters);
-    RICK_LANES(RICK_SC, 4) RICK_LANES(RICK_SC, 2) RICK_LANES(RICK_SC, 1)
+#define RICK_LANES(NN) RICK_SC(1, NN) RICK_SC(4, NN) RICK_SC(16, NN) RICK_SC(32, NN)
+    RICK_LANES(4) RICK_LANES(2) RICK_LANES(1)
+#undef RICK_LANES
 #undef RICK_SC
     RICK_CUDA(cudaGetLastError());
   }

@@ -291,9 +291,9 @@ bool batch_cached_tuning(int precision, rick_batch_tuning *t);
 
 // Samples per load of the sample pass (4, 2 or 1) for rows of nv samples in npol
 // polarisations at these addresses, and the lanes per row for rows of `per_row`
-// loads (skips: a shard that skips most rows) (bin.cu).
+// loads (bin.cu; w-plane shards have schedules of their own there).
 int sample_vector(const float *vis_re, const float *vis_im, uint64_t nv, uint32_t npol);
-int lanes_per_row(uint64_t per_row, bool skips = false);
+int lanes_per_row(uint64_t per_row);
 
 int num_sms();
 
