@@ -255,12 +255,13 @@ __device__ __forceinline__ uint32_t bin_of_item(const uint32_t *__restrict__ ite
   return lo;
 }
 
+// Items as ItemRule sizes them (the mixed form's parts capped).
 // Six blocks per SM (the launch's grid): registers bounded to 40 a thread
 // (c2 FP64 gridder 1.00 -> 0.955 ms against the compiler's own choice, five).
 template <typename OutT, int LPR, int SUP = 0>
 __global__ void __launch_bounds__(kGridThreads, 6)
     k_grid_tiles(const RecF64 *__restrict__ rec, const uint32_t *__restrict__ bin_off,
-                 const uint32_t *__restrict__ item_off, uint32_t nbins, uint32_t max_chunk,
+                 const uint32_t *__restrict__ item_off, uint32_t nbins, uint32_t fine,
                  Geometry g, int kernel, const double *__restrict__ table, int accumulate,
                  uint64_t *__restrict__ counters,
                  typename Vec2<OutT>::type *__restrict__ cube, uint32_t *__restrict__ rowmask,
@@ -299,8 +300,9 @@ __global__ void __launch_bounds__(kGridThreads, 6)
     const int tx = (int)(bin % (uint32_t)g.ntx);
     const int ty = (int)((bin / (uint32_t)g.ntx) % (uint32_t)g.nty);
     const int w = (int)(bin / ((uint32_t)g.ntx * (uint32_t)g.nty));
-    const uint32_t r0 = bin_off[bin] + chunk * max_chunk;
-    const uint32_t r1 = min(bin_off[bin + 1], r0 + max_chunk);
+    const uint32_t c0 = bin_off[bin], c1 = bin_off[bin + 1];
+    const uint32_t per = ItemRule::size<sizeof(OutT) == 4>(fine, c1 - c0);
+    const uint32_t r0 = c0 + chunk * per, r1 = min(c1, r0 + per);
     grid_item<OutT, LPR, SUP>(rec, r0, r1, g, hi, s_tab, ntab, wmax, tx, ty, w, s_nitems == 1,
                          accumulate, cube, rowmask, tilemask, &tile, s_red, &s_rows);
     __syncthreads();
@@ -434,7 +436,7 @@ __global__ void k_zero_split_tiles_batch(const BatchJob *__restrict__ jobs, int 
 
 template <typename OutT>
 int launch_grid(const Geometry &g, int kernel, Scratch &s, void *cube, int accumulate,
-                uint32_t max_chunk, cudaStream_t st, uint32_t *rowmask, uint32_t *tilemask) {
+                ItemRule rule, cudaStream_t st, uint32_t *rowmask, uint32_t *tilemask) {
   const int sms = num_sms();
   using V = typename Vec2<OutT>::type;
   const uint32_t nbins = (uint32_t)g.nbins();
@@ -443,7 +445,7 @@ int launch_grid(const Geometry &g, int kernel, Scratch &s, void *cube, int accum
   RICK_LAUNCHED();
 #define RICK_GRID(LPR, SUP)                                                                    \
   k_grid_tiles<OutT, LPR, SUP><<<blocks, kGridThreads, 0, st>>>(                               \
-      s.records, s.bin_count, s.item_off, nbins, max_chunk, g, kernel, s.table, accumulate,    \
+      s.records, s.bin_count, s.item_off, nbins, rule.fine, g, kernel, s.table, accumulate,         \
       s.counters, (V *)cube, rowmask, tilemask)
   // the common supports unrolled (7: 1.16 -> 1.00 ms FP64 at 4096^2 x 32; 9
   // with 9 lanes a record: 1.73 -> 1.20 ms at 8192^2 x 64)
@@ -463,11 +465,11 @@ int launch_grid(const Geometry &g, int kernel, Scratch &s, void *cube, int accum
 }  // namespace
 
 int grid_tiles(const Geometry &g, int kernel, int precision, Scratch &s, void *cube,
-               int accumulate, uint32_t max_chunk, cudaStream_t st, uint32_t *rowmask,
+               int accumulate, ItemRule rule, cudaStream_t st, uint32_t *rowmask,
                uint32_t *tilemask) {
   if (precision == RICK_PREC_FP64)
-    return launch_grid<double>(g, kernel, s, cube, accumulate, max_chunk, st, rowmask, tilemask);
-  return launch_grid<float>(g, kernel, s, cube, accumulate, max_chunk, st, rowmask, tilemask);
+    return launch_grid<double>(g, kernel, s, cube, accumulate, rule, st, rowmask, tilemask);
+  return launch_grid<float>(g, kernel, s, cube, accumulate, rule, st, rowmask, tilemask);
 }
 
 int zero_split_tiles(const Geometry &g, int precision, Scratch &s, void *cube, cudaStream_t st) {

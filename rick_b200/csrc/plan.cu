@@ -138,7 +138,7 @@ struct rick_plan {
   double *d_img = nullptr;     // [2*Ny*Nx] image staging for host calls
   double *d_stage = nullptr;   // conversion staging for mixed import/export
   void *d_norm = nullptr;      // NORMALIZE_UVW scratch (extrema)
-  uint32_t chunk = 1024;       // gridder records per work item of the current gridding
+  ItemRule items{1024, false};  // gridder work items of the current gridding
   // streaming ingest (rick_plan_ingest_*): rows staged in h_rows_d, samples by slices
   bool ingest = false;
   uint64_t ing_rows = 0, ing_next = 0;
@@ -258,16 +258,18 @@ int choose_fft(rick_plan *p) {
   return RICK_OK;
 }
 
-// Records per gridder work item: rows / (8 per SM), within 64..1024.  A job's dense
+// Records per gridder work item: rows / (8 per SM), within 64..1024 (more for dense
+// tiles in the mixed form, ItemRule).  A job's dense
 // tiles are split finely enough to occupy every block slot of the gridder (six an
 // SM) when rows are few -- items of 1024 left 31 of 888 slots with work at 5,418
 // rows (47 -> 14 us) and 979 for 888 at 279,800 (86 -> 65 us) -- while above 1024
 // the last items' tail grows (5.1M rows, 4096^2 x 32: 0.96 ms at 8192, 0.87 at
 // 4096, 0.80 at 1024) and below it the per-item cost does (0.81 ms at 512, 0.88 at
 // 256).
-uint32_t choose_chunk(uint64_t nrows) {
+ItemRule choose_items(uint64_t nrows, int precision) {
   const uint64_t per = nrows / ((uint64_t)num_sms() * 8);
-  return (uint32_t)std::min<uint64_t>(1024, std::max<uint64_t>(64, per));
+  return {(uint32_t)std::min<uint64_t>(1024, std::max<uint64_t>(64, per)),
+          precision == RICK_PREC_MIXED};
 }
 
 int ensure_lm(rick_plan *p, int xaxis, int yaxis, int xtot, int ytot, double resolution,
@@ -342,8 +344,8 @@ int grid_begin(rick_plan *p, uint64_t nrows, const double *uu, const double *vv,
     RICK_TRY(normalize_uvw(nrows, const_cast<double *>(uu), const_cast<double *>(vv),
                            const_cast<double *>(ww), p->d_norm, st));
   RICK_CUDA(cudaMemsetAsync(p->d_clear, 0, p->clear_bytes, st));
-  p->chunk = choose_chunk(nrows);
-  RICK_TRY(bin_count_rows(p->g, nrows, uu, vv, ww, p->s, p->chunk, st));
+  p->items = choose_items(nrows, p->d.precision);
+  RICK_TRY(bin_count_rows(p->g, nrows, uu, vv, ww, p->s, p->items, st));
   return mark(p, p->ev[1], st);
 }
 
@@ -363,7 +365,7 @@ int grid_finish(rick_plan *p, uint64_t nrows, int accumulate, bool sparse, cudaS
     RICK_CUDA(cudaMemsetAsync(p->cube, 0, p->cube_vals * p->val_bytes, st));
   }
   RICK_TRY(mark(p, p->ev[3], st));
-  RICK_TRY(grid_tiles(p->g, p->d.kernel, p->d.precision, p->s, p->cube, accumulate, p->chunk,
+  RICK_TRY(grid_tiles(p->g, p->d.kernel, p->d.precision, p->s, p->cube, accumulate, p->items,
                       st, sparse ? p->f.rowmask : nullptr, sparse ? p->f.tilemask : nullptr));
   RICK_TRY(mark(p, p->ev[4], st));
   p->ran[0] = p->ran[1] = p->ran[3] = true;
