@@ -716,15 +716,16 @@ int lanes_per_row(uint64_t per_row) {
 //   * 16 to 31: eight lanes, skipping (24 loads: 271 / 232 against 404 / 399 reading
 //     every row and 408 / 387 skipping with sixteen lanes; 309 / 301 against 410 /
 //     407 and 496 / 487 with nine tenths kept);
-//   * 8 to 15: four lanes reading every row where the shard has half of the planes or
-//     more (12 loads: 150 / 144 against 268 / 222 skipping with eight lanes); below
-//     that up to 12 loads a lane a row with block-wise places, which skips (12 loads,
-//     a quarter of the rows kept: 111 / 103 against 222 / 164), and eight lanes beyond
-//     (15 loads, a third of the planes with 0.95 of the rows: 304 against 333);
-//   * fewer: block-wise places from half of the planes on, else a lane a row with
-//     places taken by warp (4 loads, a quarter kept: 76 / 56 against 74 / 61; all but
-//     a tenth: 106 / 90 against 115 / 102, but 176 against 115 on tracks, whose dense
-//     bins the block-wise places are for).
+//   * half of the planes or more: 8 to 15 loads four lanes reading every row (12 loads:
+//     150 / 144 against 268 / 222 skipping with eight lanes), fewer a lane a row with
+//     block-wise places, which skips (4 loads, all but a tenth kept: 115 / 102 against
+//     106 / 90 with places taken by warp, but 115 against 176 on tracks, whose dense
+//     bins the block-wise places are for);
+//   * less: up to 12 loads a lane a row, skipping (12 loads, a quarter of the rows kept:
+//     128 / 109 against 222 / 164 with eight lanes; with block-wise places 111 / 103, but
+//     381 against 320 for 3.8M rows of 8 loads on 8192^2, 16 of 64 planes, where tiles
+//     share few rows), from 13 on eight lanes (15 loads, a third of the planes with 0.95
+//     of the rows: 304 against 333 with a lane a row).
 struct SampleSchedule {
   int lanes;
   bool skip;  // one lane without skip: block-wise places (k_bin_scatter_short)
@@ -732,9 +733,8 @@ struct SampleSchedule {
 static SampleSchedule shard_schedule(uint64_t per_row, bool under_half) {
   if (per_row >= 32) return {32, true};
   if (per_row >= 16) return {8, true};
-  if (per_row >= 13 && under_half) return {8, true};
-  if (per_row >= 8) return {under_half ? 1 : 4, false};
-  return {1, under_half};
+  if (under_half) return {per_row >= 13 ? 8 : 1, true};
+  return {per_row >= 8 ? 4 : 1, false};
 }
 
 // 16-byte loads where the rows start on 16 bytes and a load's polarisations repeat
