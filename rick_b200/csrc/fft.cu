@@ -448,6 +448,15 @@ template <typename S, int L> struct ColState {
   using T = std::conditional_t<kWide, double, S>;
 };
 
+// Where the sums take the steps of planes without data: pixel by pixel in the loop that
+// adds a plane, or in a loop of its own before it.  The former makes the unrolled loop
+// long, and with few warps an SM it runs at the rate its instructions are fetched (us,
+// in the loop and apart: one mixed job of 64^2 x 64 planes 265 and 163, of 512^2 x 64
+// 353 and 250, 24 of them 2,969 and 2,352; column pass of 4096^2 x 32 FP64 2,586 and
+// 2,519, of 8192^2 x 32 mixed 6,687 and 6,229); but the packed FP32 state of columns of
+// 1024 to 4096 points spills with the second (4096^2 x 32 mixed 1,303 and 1,357).
+template <typename S, int L> constexpr bool kGapInLoop = kLanes<S> == 2 && L >= 10 && L <= 12;
+
 // From 1024-point columns on the column pass leaves the sums, unit by unit, in the
 // gridded cube, which the row pass has read, and k_fft_finish applies P and turns
 // them into image rows.  Written by the column pass itself the image rows of a unit
@@ -521,8 +530,7 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
     const int m = t + G * q;
     return F::kSplit ? 2 * m + half : m;
   };
-  auto root_of = [&](int n, int m) {
-    const double l = J.ltab[n], mm = J.mtab[m];
+  auto root_of = [](double l, double mm) {
     return __dsqrt_rn(__dsub_rn(1.0, __dadd_rn(__dmul_rn(l, l), __dmul_rn(mm, mm))));
   };
   int iw = prev_plane(hi);
@@ -540,15 +548,20 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
   int nxt = prev_plane(iw);
   // sums (zero) and steps (not used by a single plane) into TMEM
   const double dwstep = __dmul_rn(twopi, J.dw);
+  // (a pixel's m is read while the one before it is worked on)
+  double l[NL], mm = J.mtab[pixel_row(0)];
+#pragma unroll
+  for (int i = 0; i < NL; i++) l[i] = J.ltab[NL * u + i];
 #pragma unroll 1
   for (int q = 0; q < kVpt; q++) {
+    const double mm_next = J.mtab[pixel_row(min(q + 1, kVpt - 1))];
     double cs[NL], sn[NL];
 #pragma unroll
     for (int i = 0; i < NL; i++) {
       cs[i] = 1.0;
       sn[i] = 0.0;
       if (phase && nxt >= lo)
-        sincos(__dmul_rn(dwstep, __dsub_rn(root_of(NL * u + i, pixel_row(q)), 1.0)), &sn[i], &cs[i]);
+        sincos(__dmul_rn(dwstep, __dsub_rn(root_of(l[i], mm), 1.0)), &sn[i], &cs[i]);
     }
 #pragma unroll
     for (int c = 0; c < M; c++) {
@@ -563,6 +576,7 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
       tm::st4(taddr + 4 * (M * q + c), z4);
       tm::st4(taddr + kStepCol + 4 * (M * q + c), w4);
     }
+    mm = mm_next;
   }
   const auto *tw = J.tw + (F::kSplit && half ? F::kTab : 0);
   // the rows a first pass takes: with L = 13, t + G r and t + G r + N combined
@@ -592,13 +606,38 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
     int tp = t;
     asm volatile("" : "+r"(tp));
     fft::first_pass<L, S>(s, tp, half, v);
+    // planes without data in between: sum * step^(gap - 1) (while no values are held)
+    const int gap = prev - iw;
+    if (!kGapInLoop<S, L> && gap > 1) {
+#pragma unroll 1
+      for (int i0 = 0; i0 < kVpt * M; i0 += 2) {
+        uint32_t sum[8], step[8];
+        tm::ld8(taddr + 4 * i0, sum);
+        tm::ld8(taddr + kStepCol + 4 * i0, step);
+        tm::wait_ld8x2(sum, step);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          A ar = tm::join<A>(sum + 4 * h), ai = tm::join<A>(sum + 4 * h + 2);
+          const A sr = tm::join<A>(step + 4 * h), si = tm::join<A>(step + 4 * h + 2);
+#pragma unroll 1
+          for (int g2 = 1; g2 < gap; g2++) {
+            const A tr = fft::fma_(ar, sr, fft::neg(fft::mul(ai, si)));
+            ai = fft::fma_(ar, si, fft::mul(ai, sr));
+            ar = tr;
+          }
+          tm::split(ar, sum + 4 * h);
+          tm::split(ai, sum + 4 * h + 2);
+        }
+        tm::st8(taddr + 4 * i0, sum);
+      }
+      tm::wait_st();
+    }
     fft::later_passes<L, S>(
         s, tp, [&](int e) { return fft::twiddle(tw + e); }, v);
     // sum = sum * step^gap + x, two pixels at a time; as their values are
     // consumed, the next plane's rows take their registers (more pixels per
     // TMEM access, or the next pair's access ahead, spill registers: 2.62 ms at
     // 4096^2 x 32 FP64 against 2.86 and more)
-    const int gap = prev - iw;
 #pragma unroll
     for (int i0 = 0; i0 < kVpt * M; i0 += 2) {
       uint32_t sum[8], step[8];
@@ -616,10 +655,12 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
           x = v[q];
         A ar = tm::join<A>(sum + 4 * h), ai = tm::join<A>(sum + 4 * h + 2);
         const A sr = tm::join<A>(step + 4 * h), si = tm::join<A>(step + 4 * h + 2);
-        for (int g2 = 1; g2 < gap; g2++) {  // planes without data in between
-          const A tr = fft::fma_(ar, sr, fft::neg(fft::mul(ai, si)));
-          ai = fft::fma_(ar, si, fft::mul(ai, sr));
-          ar = tr;
+        if constexpr (kGapInLoop<S, L>) {
+          for (int g2 = 1; g2 < gap; g2++) {  // planes without data in between
+            const A tr = fft::fma_(ar, sr, fft::neg(fft::mul(ai, si)));
+            ai = fft::fma_(ar, si, fft::mul(ai, sr));
+            ar = tr;
+          }
         }
         tm::split(fft::fma_(ar, sr, fft::fma_(fft::neg(ai), si, x.re)), sum + 4 * h);
         tm::split(fft::fma_(ar, si, fft::fma_(ai, sr, x.im)), sum + 4 * h + 2);
@@ -659,8 +700,12 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
   const double cw = __dmul_rn(twopi, __dadd_rn(J.wmin, __dmul_rn((double)(J.w_first + prev), J.dw)));
   const bool vec = NL == 2 && ((reinterpret_cast<uintptr_t>(J.img_re) |
                                 reinterpret_cast<uintptr_t>(J.img_im)) & 15u) == 0;
+  mm = J.mtab[pixel_row(0)];
+#pragma unroll
+  for (int c = 0; c < NL; c++) l[c] = J.ltab[NL * u + c];
 #pragma unroll 1
   for (int q = 0; q < kVpt; q++) {
+    const double mm_next = J.mtab[pixel_row(min(q + 1, kVpt - 1))];
     double re[NL], im[NL];
 #pragma unroll
     for (int c = 0; c < NL; c++) {
@@ -678,7 +723,7 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
       }
       double pr = 1.0, pi = 0.0;
       if (phase) {
-        const double root = root_of(NL * u + c, pixel_row(q));
+        const double root = root_of(l[c], mm);
         double sn, cs;
         sincos(__dmul_rn(cw, __dsub_rn(root, 1.0)), &sn, &cs);
         const double amp = J.dwnorm * root;
@@ -705,6 +750,7 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
         J.img_im[o + c] = im[c];
       }
     }
+    mm = mm_next;
   }
 }
 
