@@ -98,26 +98,28 @@ struct Scratch {
 
 // Records per gridder work item of a tile with c records: `fine`, but in the mixed
 // form (cap_parts) so many that a tile of more than kParts items has at most kParts of
-// up to 1024 records, or 4 kParts of up to 4096, powers of two so that the scan of
-// all bins divides by `fine` alone.  Every item is added into FP32 cells, which lose about
+// up to 1024 records, or 2 kParts of up to 4096, powers of two so that the scan of all
+// bins divides by `fine` alone.  Every item is added into FP32 cells, which lose about
 // sqrt(items / 3) of an add's rounding on the way, while the items' own 32-bit sums
 // lose the more the more records they hold (grid.cu).  Error of images against 64
-// bits, 64^2 on one plane, three array layouts: 75,000 rows 2.2, 1.8 and 1.9e-7 (3.1,
+// bits, 64^2 on one plane, three array layouts: 75,000 rows 2.1, 2.0 and 2.0e-7 (3.1,
 // 3.2 and 4.1e-7 with items of 64 throughout, 3.1, 2.5 and 2.1e-7 with 1024); 5M rows
-// 4.6, 3.7 and 3.8e-7 (6.4, 6.0 and 8.4e-7 with 1024, 8.0, 5.2 and 5.8e-7 with 8192).  FP64 cells and
+// 4.5, 3.8 and 4.1e-7 (6.4, 6.0 and 8.4e-7 with 1024, 8.0, 5.2 and 5.8e-7 with 8192).
+// Half as many parts cost time where a tile holds much of a job (100,000 rows, 1024^2,
+// one plane, support 15: 234 us a call against 178, and 161 uncapped).  FP64 cells and
 // sums lose nothing that shows.
 struct ItemRule {
-  static constexpr uint32_t kParts = 64;
+  static constexpr uint32_t kParts = 128;
   uint32_t fine;  // at most 1024 with cap_parts
   bool cap_parts;
-  // log2 of the size of a capped tile's items: c / 64 up to 1024, or c / 256 up to 4096
+  // log2 of the size of a capped tile's items: c / 128 up to 1024, or c / 256 up to 4096
   // where that is more, rounded up to powers of two
   static __device__ __forceinline__ uint32_t size_log(uint32_t c) {
-    const uint32_t part = 32 - __clz((c - 1) / kParts), few = 32 - __clz((c - 1) / (4 * kParts));
+    const uint32_t part = 32 - __clz((c - 1) / kParts), few = 32 - __clz((c - 1) / (2 * kParts));
     return max(min(part, 10u), min(few, 12u));
   }
   template <bool CAP> static __device__ __forceinline__ bool capped(uint32_t fine, uint32_t c) {
-    return CAP && c > kParts * fine;  // c > 4096
+    return CAP && c > kParts * fine;  // c > 8192
   }
   template <bool CAP> static __device__ __forceinline__ uint32_t size(uint32_t fine, uint32_t c) {
     return capped<CAP>(fine, c) ? 1u << size_log(c) : fine;

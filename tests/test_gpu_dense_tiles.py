@@ -18,7 +18,7 @@ def _one_tile(n, nx, lo, hi):
             rng.standard_normal(n).astype(np.float32)]
 
 
-@pytest.mark.parametrize("n", [63, 64, 65, 1024, 4096, 4097, 16400, 65537, 262145])
+@pytest.mark.parametrize("n", [63, 64, 65, 1024, 8192, 8193, 16400, 131073, 262145])
 @pytest.mark.parametrize("nx", [64, 50])
 def test_item_sizes(nx, n):
     """Below and above the sizes at which a tile is split and its items grow."""
@@ -32,10 +32,10 @@ def test_item_sizes(nx, n):
         assert (st["work_items"] > 1) == (n > 64)
 
 
-@pytest.mark.parametrize("n,items", [(4000, 63), (5000, 40), (75_000, 74), (600_000, 147)])
+@pytest.mark.parametrize("n,items", [(8000, 125), (10_000, 79), (75_000, 74), (600_000, 147)])
 def test_parts_added_into_fp32_cells(n, items):
     """Each item of a tile is added into its cells: in the mixed form, whose cells are
-    FP32, at most 64 of fewer than 1024 records, and 256 of more."""
+    FP32, at most 128 of fewer than 1024 records, and 256 of more."""
     host = _one_tile(n, 64, 8, 23)
     _, st = gpu_grid(gpu_rows(*host), n, 64, 64, 1, 7, "gauss", 1, 1, "mixed", R.ROWS_ALL)
     assert st["work_items"] == items
