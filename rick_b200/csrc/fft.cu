@@ -548,19 +548,20 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
   int nxt = prev_plane(iw);
   // sums (zero) and steps (not used by a single plane) into TMEM
   const double dwstep = __dmul_rn(twopi, J.dw);
+  const bool steps = phase && nxt >= lo;
   // (a pixel's m is read while the one before it is worked on)
-  double l[NL], mm = J.mtab[pixel_row(0)];
+  double l[NL], mm = steps ? J.mtab[pixel_row(0)] : 0.0;
 #pragma unroll
-  for (int i = 0; i < NL; i++) l[i] = J.ltab[NL * u + i];
+  for (int i = 0; i < NL; i++) l[i] = steps ? J.ltab[NL * u + i] : 0.0;
 #pragma unroll 1
   for (int q = 0; q < kVpt; q++) {
-    const double mm_next = J.mtab[pixel_row(min(q + 1, kVpt - 1))];
+    const double mm_next = steps ? J.mtab[pixel_row(min(q + 1, kVpt - 1))] : 0.0;
     double cs[NL], sn[NL];
 #pragma unroll
     for (int i = 0; i < NL; i++) {
       cs[i] = 1.0;
       sn[i] = 0.0;
-      if (phase && nxt >= lo)
+      if (steps)
         sincos(__dmul_rn(dwstep, __dsub_rn(root_of(l[i], mm), 1.0)), &sn[i], &cs[i]);
     }
 #pragma unroll
@@ -700,12 +701,12 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
   const double cw = __dmul_rn(twopi, __dadd_rn(J.wmin, __dmul_rn((double)(J.w_first + prev), J.dw)));
   const bool vec = NL == 2 && ((reinterpret_cast<uintptr_t>(J.img_re) |
                                 reinterpret_cast<uintptr_t>(J.img_im)) & 15u) == 0;
-  mm = J.mtab[pixel_row(0)];
+  mm = phase ? J.mtab[pixel_row(0)] : 0.0;
 #pragma unroll
-  for (int c = 0; c < NL; c++) l[c] = J.ltab[NL * u + c];
+  for (int c = 0; c < NL; c++) l[c] = phase ? J.ltab[NL * u + c] : 0.0;
 #pragma unroll 1
   for (int q = 0; q < kVpt; q++) {
-    const double mm_next = J.mtab[pixel_row(min(q + 1, kVpt - 1))];
+    const double mm_next = phase ? J.mtab[pixel_row(min(q + 1, kVpt - 1))] : 0.0;
     double re[NL], im[NL];
 #pragma unroll
     for (int c = 0; c < NL; c++) {
