@@ -283,9 +283,12 @@ typedef struct rick_job_desc {
 } rick_job_desc;
 
 /* Schedule knobs of a batch: gridder records per work item and gridder blocks
- * per SM.  planes_in_flight (0, 1 or 2) is kept as given and selects nothing: the
- * column pass has one form, each pixel's running sum and w-step in tensor memory
- * (one plane per iteration). */
+ * per SM; planes_in_flight chooses how the column pass sums the planes: 0 all of
+ * them under one recurrence of the w-correction's factor; 1 or 2 (no difference
+ * between them) in groups of eight with a factor formed anew for each, which
+ * keeps the recurrence's rounding from adding up over many planes (FP64 jobs of
+ * more than 8 planes, mixed ones of more than 16 with 1024 rows and more; a
+ * little slower).  The autotuner takes 0, servers take 1. */
 typedef struct rick_batch_tuning {
   uint32_t max_chunk;
   int grid_blocks_per_sm;

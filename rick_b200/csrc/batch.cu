@@ -187,6 +187,7 @@ namespace {
 // The launch sequence of one batch run (stream-ordered; captured in the graph).
 int batch_launch(rick_batch *b, cudaStream_t st) {
   b->bl.grid_blocks_per_sm = b->tune.grid_blocks_per_sm;
+  b->fj.anchored = b->tune.planes_in_flight > 0;
   RICK_CUDA(cudaMemsetAsync(b->arena + b->L.clear, 0, b->L.clear_bytes, st));
   RICK_TRY(bin_rows_batch(b->bl, b->s, b->tune.max_chunk, st));
   RICK_TRY(grid_tiles_batch(b->bl, b->precision, b->s, b->tune.max_chunk, st));

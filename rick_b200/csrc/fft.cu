@@ -482,16 +482,68 @@ template <typename S> struct ColJob {
   const double *ltab, *mtab;
   double wmin, dw, dwnorm, norm;
   int phase_on;
+  int anchor;                      // planes of a group with a factor of its own (kAnchored)
   double *img_re, *img_im;
-  typename Vec<S>::t *sums;        // [units][ny], L = 13: [units][half][ny / 2] (kFinish)
+  typename Vec<S>::t *sums;        // [units][ny], L = 13: [units][half][ny / 2] (kFinish, groups)
 };
+
+// The column pass of a batch whose schedule asks for it (planes_in_flight 1 or 2, a
+// server's) sums groups of kAnchorPlanes planes by themselves, each group's factor
+// formed anew from its lowest plane: the steps' rounding otherwise adds up over all
+// planes.  Off the 64-bit image in one sum / by groups: mixed 1024^2 x 64 planes 7.1e-7 /
+// 2.6e-7 (one job 394 / 511 us), 2048^2 x 24 3.6e-7 / 2.7e-7 (473 / 563 us); FP64 1024^2
+// x 16 1.5e-14 / 1.0e-14 (257 / 267 us), 512^2 x 64 7.4e-15 / 4.5e-15 (281 / 357 us).
+// FP32 sums of up to kPlainPlanes planes are left whole: the transforms' own error is
+// the larger there.
+constexpr int kAnchorPlanes = 8, kPlainPlanes = 16;
+template <typename S, int L> constexpr bool kAnchored = kLanes<S> == 1 || L >= 10;
+template <typename S> __host__ __device__ constexpr int plain_planes() {
+  return kLanes<S> == 1 ? kAnchorPlanes : kPlainPlanes;
+}
+
+// sum += total * (factor of plane `from` / factor of plane `to`) for one pixel with root
+// minus one rm1 (of each lane): the sum of the groups above, down to plane `from`, joins
+// that of the group whose lowest plane is `to`.
+template <typename S>
+__device__ __forceinline__ void join_groups(uint32_t *sum, Cx<S> total, const ColJob<S> &J, int from,
+                                            int to, const double (&rm1)[kLanes<S>]) {
+  const double twopi = 2.0 * kPi;
+  auto turn = [&](int w, double rootm1) {
+    return __dmul_rn(__dmul_rn(twopi, __dadd_rn(J.wmin, __dmul_rn((double)(J.w_first + w), J.dw))),
+                     rootm1);
+  };
+  double er[kLanes<S>], ei[kLanes<S>];
+#pragma unroll
+  for (int c = 0; c < kLanes<S>; c++) {
+    // the difference of the two rounded arguments, and what it leaves (two-sum)
+    const double a = turn(from, rm1[c]), b = turn(to, rm1[c]);
+    const double d = __dsub_rn(a, b), bb = __dsub_rn(a, d);
+    const double rest = __dsub_rn(__dsub_rn(a, __dadd_rn(d, bb)), __dsub_rn(b, bb));
+    double sn, cs;
+    sincos(d, &sn, &cs);
+    er[c] = fma(-rest, sn, cs);
+    ei[c] = fma(rest, cs, sn);
+  }
+  const S ar = tm::join<S>(sum), ai = tm::join<S>(sum + 2);
+  if constexpr (kLanes<S> == 2) {
+    const auto re = [](double x, double y, double c, double s, double a) { return (float)fma(x, c, fma(-y, s, a)); };
+    const auto im = [](double x, double y, double c, double s, double a) { return (float)fma(x, s, fma(y, c, a)); };
+    tm::split(make_float2(re(total.re.x, total.im.x, er[0], ei[0], ar.x),
+                          re(total.re.y, total.im.y, er[1], ei[1], ar.y)), sum);
+    tm::split(make_float2(im(total.re.x, total.im.x, er[0], ei[0], ai.x),
+                          im(total.re.y, total.im.y, er[1], ei[1], ai.y)), sum + 2);
+  } else {
+    tm::split(fma(total.re, er[0], fma(-total.im, ei[0], ar)), sum);
+    tm::split(fma(total.re, ei[0], fma(total.im, er[0], ai)), sum + 2);
+  }
+}
 
 // Unit u of one job, column u or columns 2u, 2u + 1 (with L = 13, half `half` of
 // its pixels), over the planes lo..hi-1, by the group's thread t; the result is
 // stored in the image, or (add) added to it.  taddr: the thread's TMEM address,
 // pixel q's sum at 4 q (wide state: at 8 q, column by column) and its step kStepCol
 // further.
-template <typename S, int L>
+template <typename S, int L, bool ANCHOR = false>
 __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, int half, int lo,
                                              int hi, bool add, int t, const ColJob<S> &J,
                                              uint32_t taddr) {
@@ -598,6 +650,18 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
   uint32_t nbits = nxt >= lo ? row_bits(nxt) : 0u;
   int prev = iw;
   tm::wait_st();
+  // ANCHOR: the sum of the groups done, in the place of the job's column sums
+  V *total = J.sums + (uint64_t)u * ny + t;
+  int lowest = lo, done = -1;  // done: lowest plane of the groups in `total`
+  if constexpr (ANCHOR)
+    while (__ldg(counts + 1 + lowest) == 0) lowest++;
+  auto joined = [&](int q, uint32_t (&sum)[4], int to) {
+    double rm1[NL];
+#pragma unroll
+    for (int c = 0; c < NL; c++)
+      rm1[c] = __dsub_rn(root_of(J.ltab[NL * u + c], J.mtab[pixel_row(q)]), 1.0);
+    join_groups<S>(sum, fft::unpack(total[G * q]), J, done, to, rm1);
+  };
   for (;;) {
     col = plane_rows(nxt >= lo ? nxt : iw);
     const int nxt2 = nxt >= lo ? prev_plane(nxt) : nxt;
@@ -607,6 +671,22 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
     int tp = t;
     asm volatile("" : "+r"(tp));
     fft::first_pass<L, S>(s, tp, half, v);
+    if constexpr (ANCHOR) {
+      if (phase && (prev - lowest) / J.anchor != (iw - lowest) / J.anchor) {
+        // plane prev was the lowest of its group (no values are held here)
+#pragma unroll 1
+        for (int q = 0; q < kVpt; q++) {
+          uint32_t sum[4], zero[4] = {0, 0, 0, 0};
+          tm::ld4(taddr + 4 * q, sum);
+          tm::wait_ld4(sum);
+          tm::st4(taddr + 4 * q, zero);
+          if (done >= 0) joined(q, sum, prev);
+          total[G * q] = fft::pack(Cx<S>{tm::join<S>(sum), tm::join<S>(sum + 2)});
+        }
+        tm::wait_st();
+        done = prev;
+      }
+    }
     // planes without data in between: sum * step^(gap - 1) (while no values are held)
     const int gap = prev - iw;
     if (!kGapInLoop<S, L> && gap > 1) {
@@ -692,6 +772,9 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
         uint32_t a4[4];
         tm::ld4(taddr + 4 * q, a4);
         tm::wait_ld4(a4);
+        if constexpr (ANCHOR) {
+          if (done >= 0) joined(q, a4, prev);
+        }
         to[G * q] = fft::pack(Cx<S>{tm::join<S>(a4), tm::join<S>(a4 + 2)});
       }
       return;
@@ -714,6 +797,9 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
       uint32_t a4[4];
       tm::ld4(taddr + 4 * (M * q + (CS::kWide ? c : 0)), a4);
       tm::wait_ld4(a4);
+      if constexpr (ANCHOR) {
+        if (done >= 0) joined(q, a4, prev);
+      }
       const A sr = tm::join<A>(a4), si = tm::join<A>(a4 + 2);
       if constexpr (kLanes<A> == 2) {
         ar = c ? sr.y : sr.x;
@@ -818,8 +904,8 @@ __global__ void __launch_bounds__(Shape<L>::kThreads, col_blocks<S, L>()) k_fft_
 
 // The column pass over the jobs col_jobs[lo..hi-1] of a batch (all of FFT length
 // 2^L along y): the blocks' worths of units of the k-th listed job are
-// col_units[k] .. col_units[k+1]-1.
-template <typename S, int L>
+// col_units[k] .. col_units[k+1]-1.  ANCHOR: factors formed anew (kAnchored).
+template <typename S, int L, bool ANCHOR>
 __global__ void __launch_bounds__(Shape<L>::kThreads, col_blocks<S, L>())
     k_fft_cols_multi(const BatchJob *__restrict__ jobs, const uint32_t *__restrict__ col_jobs,
                      int lo, int hi, const uint32_t *__restrict__ col_units,
@@ -857,12 +943,13 @@ __global__ void __launch_bounds__(Shape<L>::kThreads, col_blocks<S, L>())
       J.dwnorm = B.dwnorm;
       J.norm = B.norm;
       J.phase_on = B.phase_on;
+      J.anchor = B.g.nw > plain_planes<S>() ? kAnchorPlanes : B.g.nw;
       J.img_re = B.img_re;
       J.img_im = B.img_im;
       J.sums = (V *)B.cube;
     }
     __syncthreads();
-    fft_col_unit<S, L>(s, s_unit + grp, 0, 0, sJ.nw, false, t, sJ, tmem.addr);
+    fft_col_unit<S, L, ANCHOR>(s, s_unit + grp, 0, 0, sJ.nw, false, t, sJ, tmem.addr);
   }
   tmem.release();
 }
@@ -1083,6 +1170,7 @@ template <typename S> ColJob<S> col_job(const BatchJob &B, const FftJobs &f) {
   J.dwnorm = B.dwnorm;
   J.norm = B.norm;
   J.phase_on = B.phase_on;
+  J.anchor = 0;  // (a plan's factors: one product over all planes)
   J.img_re = B.img_re;
   J.img_im = B.img_im;
   J.sums = (typename Vec<S>::t *)B.cube;
@@ -1138,9 +1226,13 @@ int launch_cols(const FftJobs &f, const FftClass &c, cudaStream_t st) {
   const size_t floor_b = (size_t)smem_sm / (size_t)(max_blocks + 1) + 1;
   if (sm + (size_t)reserved < floor_b) sm = floor_b - (size_t)reserved;
   sm = (sm + 15) & ~(size_t)15;
+  const bool anchor = f.anchored && c.planes > plain_planes<S>() && kAnchored<S, L>;
   const void *fn = (const void *)k_fft_cols<S, L>;
   if constexpr (L <= kMultiMaxLog) {
-    if (!f.one) fn = (const void *)k_fft_cols_multi<S, L>;
+    if (!f.one) fn = (const void *)k_fft_cols_multi<S, L, false>;
+    if constexpr (kAnchored<S, L>) {
+      if (!f.one && anchor) fn = (const void *)k_fft_cols_multi<S, L, true>;
+    }
   }
   RICK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   // a shared-memory carveout just large enough for those blocks: the rest of the
@@ -1166,8 +1258,14 @@ int launch_cols(const FftJobs &f, const FftClass &c, cudaStream_t st) {
     }
   } else if constexpr (L <= kMultiMaxLog) {
     const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(c.units, slots));
-    k_fft_cols_multi<S, L><<<blocks, BT, sm, st>>>(f.jobs, f.col_jobs, c.lo, c.hi, f.col_units,
-                                                   f.rowbits, f.counts);
+    if (anchor) {
+      if constexpr (kAnchored<S, L>)
+        k_fft_cols_multi<S, L, true><<<blocks, BT, sm, st>>>(f.jobs, f.col_jobs, c.lo, c.hi,
+                                                             f.col_units, f.rowbits, f.counts);
+    } else {
+      k_fft_cols_multi<S, L, false><<<blocks, BT, sm, st>>>(f.jobs, f.col_jobs, c.lo, c.hi,
+                                                            f.col_units, f.rowbits, f.counts);
+    }
     if constexpr (kFinish<L>) {
       RICK_LAUNCHED();
       const uint64_t tiles = c.units * (uint64_t)(kLanes<S> * F::kGroups * (1 << L) / (2 * kTile * kTile));
@@ -1228,7 +1326,7 @@ void fft_classes(const BatchJob *jobs, int njobs, int precision, FftJobs &f, uin
   f.n_row_cls = 0;
   for (int j = 0; j < njobs; j++) {
     if (f.n_row_cls == 0 || f.row_cls[f.n_row_cls - 1].log != jobs[j].logx)
-      f.row_cls[f.n_row_cls++] = FftClass{jobs[j].logx, j, j + 1, 0};
+      f.row_cls[f.n_row_cls++] = FftClass{jobs[j].logx, j, j + 1, 0, 0};
     else
       f.row_cls[f.n_row_cls - 1].hi = j + 1;
   }
@@ -1241,6 +1339,7 @@ void fft_classes(const BatchJob *jobs, int njobs, int precision, FftJobs &f, uin
   for (int l = 6; l <= 13; l++) {
     const int lo = n;
     uint32_t units = 0;
+    int planes = 0;
     for (int j = 0; j < njobs; j++) {
       if (jobs[j].logy != l) continue;
       col_jobs[n] = (uint32_t)j;
@@ -1248,9 +1347,10 @@ void fft_classes(const BatchJob *jobs, int njobs, int precision, FftJobs &f, uin
       const uint32_t u = (uint32_t)jobs[j].g.nx / lanes / (uint32_t)fft_groups_per_block(l);
       acc += u;
       units += u;
+      planes = std::max(planes, jobs[j].g.nw);
       n++;
     }
-    if (n > lo) f.col_cls[f.n_col_cls++] = FftClass{l, lo, n, units};
+    if (n > lo) f.col_cls[f.n_col_cls++] = FftClass{l, lo, n, units, planes};
   }
   col_units[n] = acc;
 }

@@ -180,6 +180,7 @@ struct FftClass {
   int log;         // log2 of the FFT length
   int lo, hi;      // jobs[lo..hi) (row pass) or col_jobs[lo..hi) (column pass)
   uint32_t units;  // column groups of the class (column pass)
+  int planes;      // most planes of a job of the class (column pass)
 };
 struct FftJobs {
   const BatchJob *jobs = nullptr;    // device [njobs]
@@ -192,6 +193,7 @@ struct FftJobs {
   uint32_t *rowmask = nullptr, *tilemask = nullptr, *rowlist = nullptr, *counts = nullptr;
   uint16_t *rowbits = nullptr;          // two entries per row-mask word
   int cols_parts = 1;                   // blocks a unit's planes are dealt to (one job)
+  bool anchored = false;                // factors formed anew along the planes (a batch)
   int n_row_cls = 0, n_col_cls = 0;
   FftClass row_cls[8], col_cls[8];
   // a set of one job (a plan): its host copy; the FFT kernels then take the

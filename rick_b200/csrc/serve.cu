@@ -74,7 +74,7 @@ struct rick_server {
   // blocks allocate tensor memory; see rick_batch::cols_gate); batches are
   // launched by the scheduler thread alone, in order
   cudaEvent_t cols_gate = nullptr;
-  rick_batch_tuning tune{2048, 6, 0};
+  rick_batch_tuning tune{2048, 6, 1};
   rick_server_stats stats{};
 };
 
@@ -271,6 +271,7 @@ int rick_server_create(rick_server **out, const rick_server_desc *d) {
   cudaSetDevice(s->d.device);
   rick_batch_tuning t;
   if (batch_cached_tuning(d->precision, &t)) s->tune = t;
+  s->tune.planes_in_flight = 1;  // images do not depend on what was tuned before
   cudaMemPoolProps props{};
   props.allocType = cudaMemAllocationTypePinned;
   props.location.type = cudaMemLocationTypeDevice;
