@@ -453,7 +453,7 @@ template <typename S, int L> struct ColState {
 // long, and with few warps an SM it runs at the rate its instructions are fetched (us,
 // in the loop and apart: one mixed job of 64^2 x 64 planes 265 and 163, of 512^2 x 64
 // 353 and 250, 24 of them 2,969 and 2,352; column pass of 4096^2 x 32 FP64 2,586 and
-// 2,519, of 8192^2 x 32 mixed 6,687 and 6,229); but the packed FP32 state of columns of
+// 2,519, of 8192^2 x 32 mixed 6,687 and 6,320); but the packed FP32 state of columns of
 // 1024 to 4096 points spills with the second (4096^2 x 32 mixed 1,303 and 1,357).
 template <typename S, int L> constexpr bool kGapInLoop = kLanes<S> == 2 && L >= 10 && L <= 12;
 
@@ -600,22 +600,7 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
   int nxt = prev_plane(iw);
   // sums (zero) and steps (not used by a single plane) into TMEM
   const double dwstep = __dmul_rn(twopi, J.dw);
-  const bool steps = phase && nxt >= lo;
-  // (a pixel's m is read while the one before it is worked on)
-  double l[NL], mm = steps ? J.mtab[pixel_row(0)] : 0.0;
-#pragma unroll
-  for (int i = 0; i < NL; i++) l[i] = steps ? J.ltab[NL * u + i] : 0.0;
-#pragma unroll 1
-  for (int q = 0; q < kVpt; q++) {
-    const double mm_next = steps ? J.mtab[pixel_row(min(q + 1, kVpt - 1))] : 0.0;
-    double cs[NL], sn[NL];
-#pragma unroll
-    for (int i = 0; i < NL; i++) {
-      cs[i] = 1.0;
-      sn[i] = 0.0;
-      if (steps)
-        sincos(__dmul_rn(dwstep, __dsub_rn(root_of(l[i], mm), 1.0)), &sn[i], &cs[i]);
-    }
+  auto set_state = [&](int q, const double (&cs)[NL], const double (&sn)[NL]) {
 #pragma unroll
     for (int c = 0; c < M; c++) {
       Cx<A> st;
@@ -629,7 +614,30 @@ __device__ __forceinline__ void fft_col_unit(typename Vec<S>::t *s, uint32_t u, 
       tm::st4(taddr + 4 * (M * q + c), z4);
       tm::st4(taddr + kStepCol + 4 * (M * q + c), w4);
     }
-    mm = mm_next;
+  };
+  double l[NL], mm = 0.0, cs[NL], sn[NL];
+#pragma unroll
+  for (int i = 0; i < NL; i++) {
+    cs[i] = 1.0;
+    sn[i] = l[i] = 0.0;
+  }
+  if (phase && nxt >= lo) {
+    // (a pixel's m is read while the one before it is worked on)
+    mm = J.mtab[pixel_row(0)];
+#pragma unroll
+    for (int i = 0; i < NL; i++) l[i] = J.ltab[NL * u + i];
+#pragma unroll 1
+    for (int q = 0; q < kVpt; q++) {
+      const double mm_next = J.mtab[pixel_row(min(q + 1, kVpt - 1))];
+#pragma unroll
+      for (int i = 0; i < NL; i++)
+        sincos(__dmul_rn(dwstep, __dsub_rn(root_of(l[i], mm), 1.0)), &sn[i], &cs[i]);
+      set_state(q, cs, sn);
+      mm = mm_next;
+    }
+  } else {
+#pragma unroll 1
+    for (int q = 0; q < kVpt; q++) set_state(q, cs, sn);
   }
   const auto *tw = J.tw + (F::kSplit && half ? F::kTab : 0);
   // the rows a first pass takes: with L = 13, t + G r and t + G r + N combined
@@ -955,12 +963,11 @@ __global__ void __launch_bounds__(Shape<L>::kThreads, col_blocks<S, L>())
 }
 
 // image = norm * P * sum, P the factor of the lowest plane with data, from the sums
-// of a column pass with 2^L rows: 32 columns by 32 rows m below ny / 2 and their
-// mirror images ny - m (ny / 2 for m = 0) a block, read along the columns (512 bytes a
-// warp) and written along the rows.  FP64 sums and the image cross HBM once, 32 bytes
-// a pixel (0.083 ms at 4096^2); a sincos and a root a pixel take as long, so rows m
-// and ny - m, whose m^2 and with it P agree on a table of equal halves, share them
-// (523 -> 461 us for the 2048-row jobs of a mixed batch of 64).
+// of a column pass with 2^L rows: 32 columns by 64 rows a block, read along the columns
+// (512 bytes a warp) and written along the rows.  FP64 sums and the image cross HBM once,
+// 32 bytes a pixel (0.083 ms at 4096^2); a sincos and a root a pixel take as long, and
+// 64 rows a block keep more of them in flight than 32 (523 -> 423 us for the 2048-row
+// jobs of a mixed batch of 64).
 constexpr int kTile = 32;
 template <typename S> using FinishTile = typename Vec<S>::t[2][kTile / kLanes<S>][kTile + 1];
 template <typename S, int L>
@@ -969,10 +976,9 @@ __device__ __forceinline__ void finish_tile(FinishTile<S> &tile, uint32_t n0, ui
   constexpr int NL = kLanes<S>;
   const uint32_t lane = threadIdx.x % 32, warp = threadIdx.x / 32, warps = blockDim.x / 32;
   const uint32_t ny = (uint32_t)J.ny;
-  auto mirror = [&](uint32_t m) { return m ? ny - m : ny / 2; };
   if (low < J.nw) {
     auto at = [](uint32_t m) { return Shape<L>::kSplit ? m % 2 * Shape<L>::N + m / 2 : m; };
-    const uint32_t at0 = at(m0 + lane), at1 = at(mirror(m0 + lane));
+    const uint32_t at0 = at(m0 + lane), at1 = at(m0 + kTile + lane);
 #pragma unroll 4
     for (uint32_t i = warp; i < kTile / NL; i += warps) {
       const typename Vec<S>::t *from = J.sums + (uint64_t)(n0 / NL + i) * ny;
@@ -985,39 +991,35 @@ __device__ __forceinline__ void finish_tile(FinishTile<S> &tile, uint32_t n0, ui
   const double cw = __dmul_rn(2.0 * kPi, __dadd_rn(J.wmin, __dmul_rn((double)(J.w_first + low), J.dw)));
   const double l = J.ltab[n0 + lane], l2 = __dmul_rn(l, l);
 #pragma unroll 1
-  for (uint32_t i = warp; i < kTile; i += warps) {
-    double mm = -1.0, pr = 1.0, pi = 0.0;
-#pragma unroll 1
-    for (int h = 0; h < 2; h++) {
-      const uint32_t m = h ? mirror(m0 + i) : m0 + i;
-      double re = 0.0, im = 0.0;
-      if (low < J.nw) {
-        const double m2 = __dmul_rn(J.mtab[m], J.mtab[m]);
-        if (phase && m2 != mm) {
-          const double root = __dsqrt_rn(__dsub_rn(1.0, __dadd_rn(l2, m2)));
-          double sn, cs;
-          sincos(__dmul_rn(cw, __dsub_rn(root, 1.0)), &sn, &cs);
-          const double amp = J.dwnorm * root;
-          pr = cs * amp;
-          pi = sn * amp;
-          mm = m2;
-        }
-        const Cx<S> x = fft::unpack(tile[h][lane / NL][i]);
-        double ar, ai;
-        if constexpr (NL == 2) {
-          ar = lane % 2 ? x.re.y : x.re.x;
-          ai = lane % 2 ? x.im.y : x.im.x;
-        } else {
-          ar = x.re;
-          ai = x.im;
-        }
-        re = J.norm * fma(ar, pr, -ai * pi);
-        im = J.norm * fma(ar, pi, ai * pr);
+  for (uint32_t i = warp; i < 2 * kTile; i += warps) {
+    const uint32_t m = m0 + i;
+    double re = 0.0, im = 0.0;
+    if (low < J.nw) {
+      double pr = 1.0, pi = 0.0;
+      if (phase) {
+        const double mm = J.mtab[m];
+        const double root = __dsqrt_rn(__dsub_rn(1.0, __dadd_rn(l2, __dmul_rn(mm, mm))));
+        double sn, cs;
+        sincos(__dmul_rn(cw, __dsub_rn(root, 1.0)), &sn, &cs);
+        const double amp = J.dwnorm * root;
+        pr = cs * amp;
+        pi = sn * amp;
       }
-      const uint64_t o = (uint64_t)m * (uint32_t)J.nx + n0 + lane;
-      __stcs(J.img_re + o, re);
-      __stcs(J.img_im + o, im);
+      const Cx<S> x = fft::unpack(tile[i / kTile][lane / NL][i % kTile]);
+      double ar, ai;
+      if constexpr (NL == 2) {
+        ar = lane % 2 ? x.re.y : x.re.x;
+        ai = lane % 2 ? x.im.y : x.im.x;
+      } else {
+        ar = x.re;
+        ai = x.im;
+      }
+      re = J.norm * fma(ar, pr, -ai * pi);
+      im = J.norm * fma(ar, pi, ai * pr);
     }
+    const uint64_t o = (uint64_t)m * (uint32_t)J.nx + n0 + lane;
+    __stcs(J.img_re + o, re);
+    __stcs(J.img_im + o, im);
   }
 }
 
@@ -1038,7 +1040,7 @@ __global__ void __launch_bounds__(kFinishThreads) k_fft_finish(ColJob<S> J) {
   __shared__ FinishTile<S> tile;
   const uint32_t across = (uint32_t)J.nx / kTile;
   const int low = lowest_plane(J.counts, J.nw);
-  finish_tile<S, L>(tile, blockIdx.x % across * kTile, blockIdx.x / across * kTile, low, J);
+  finish_tile<S, L>(tile, blockIdx.x % across * kTile, blockIdx.x / across * (2 * kTile), low, J);
 }
 
 // Of the jobs col_jobs[lo..hi-1] of a batch: a block's worth of units holds
@@ -1070,7 +1072,7 @@ __global__ void __launch_bounds__(kFinishThreads)
   J.sums = (typename Vec<S>::t *)B.cube;
   const uint32_t i = blockIdx.x - (col_units[k] - col_units[lo]) * per_block;
   const uint32_t across = (uint32_t)J.nx / kTile;
-  finish_tile<S, L>(tile, i % across * kTile, i / across * kTile,
+  finish_tile<S, L>(tile, i % across * kTile, i / across * (2 * kTile),
                     lowest_plane(counts + B.counts_base, J.nw), J);
 }
 
