@@ -65,3 +65,30 @@ def test_half_shard_leaves_the_other_half_unread():
             ms[planes] = sorted(t)[len(t) // 2]
     for planes in ((0, nw // 2), (nw // 2, nw // 2)):
         assert ms[planes] < 0.85 * ms[None], ms
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_shards_of_finished_columns(precision):
+    """Columns of 1024 rows, whose sums a finishing kernel turns into the image with the
+    factor of a shard's own lowest plane: the shards' images add up to the oracle's."""
+    import torch
+    from _util import TOL_MIXED
+    from test_gpu_sparse_fft import _oracle_image
+    nx, nw, n = 1024, 6, 900
+    rng = np.random.default_rng(3)
+    host = (rng.random(n) * 0.999, rng.random(n) * 0.999, rng.random(n) * 0.999,
+            rng.uniform(0.5, 1.5, 2 * n).astype(np.float32),
+            rng.standard_normal(2 * n).astype(np.float32),
+            rng.standard_normal(2 * n).astype(np.float32))
+    res, wmin, wmax = 1.0 / (2.4 * nx), -310.0, 290.0
+    want = np.concatenate(_oracle_image(host, nx, nx, nw, "gauss", 7, 1, 2, res, wmin, wmax))
+    rows = gpu_rows(*host)
+    total = np.zeros(2 * nx * nx)
+    for planes in ((0, 2), (2, 3), (5, 1)):
+        with R.Plan(R.Geometry(nx, nx, nw, 7, "gauss", precision), n, 1, 2, device=0,
+                    planes=planes) as plan:
+            img = torch.empty(2, nx * nx, dtype=torch.float64, device="cuda")
+            plan.image(n, rows, res, wmin, wmax, img[0], img[1], R.ROWS_ALL)
+            torch.cuda.synchronize()
+            total += img.cpu().numpy().ravel()
+    assert rel_l2(total, want) < (TOL_FP64 if precision == "fp64" else TOL_MIXED)
