@@ -39,7 +39,7 @@ template <> struct Vec2<float> { using type = float2; };
 // word with the high part.  The mixed form, whose tiles are FP32, keeps one
 // 32-bit word (resolution 2^-30 of the item's bound, finer than FP32 rounding
 // of the cells that matter).  Integer sums do not depend on the order of the
-// adds, so a tile's sum is reproducible.
+// adds, so an item's sum is reproducible (a tile's, if it is one item).
 struct FixTile {
   uint32_t lo_re[kTile * kPitch], hi_re[kTile * kPitch];
   uint32_t lo_im[kTile * kPitch], hi_im[kTile * kPitch];

@@ -1,7 +1,8 @@
 // Plan object: device-resident imaging pipeline (binning -> gridding -> FFT ->
 // w-correction) with all scratch, the w-plane cube and the cuFFT plan held
-// across calls.  Every call is stream-ordered; none synchronises the host
-// except rick_plan_image_host and rick_plan_get_stats.
+// across calls.  Every call is stream-ordered; none synchronises the host except
+// rick_plan_image_host, the end of an ingest, the stage timers, rick_plan_get_stats,
+// and the first image or phase call with another resolution (ensure_lm).
 #include <math.h>
 #include <stdarg.h>
 #include <stdlib.h>
