@@ -684,7 +684,7 @@ __global__ void __launch_bounds__(kShortThreads, 2)
 // Pass 1 and the offsets: histogram of records per bin over all rows, bin
 // offsets and work-item offsets (records are not written yet).
 int bin_count_rows(const Geometry &g, uint64_t nrows, const double *uu, const double *vv,
-                   const double *ww, Scratch &s, ItemRule rule, cudaStream_t st) {
+                   const double *ww, Scratch &s, uint32_t max_chunk, cudaStream_t st) {
   const uint64_t nbins = g.nbins();
   if (nrows == 0) {
     RICK_CUDA(cudaMemsetAsync(s.item_off, 0, (nbins + 1) * sizeof(uint32_t), st));
@@ -697,7 +697,7 @@ int bin_count_rows(const Geometry &g, uint64_t nrows, const double *uu, const do
   RICK_LAUNCHED();
   k_bin_count<<<blocks, 256, 0, st>>>(uu, vv, ww, nrows, g, s.bin_count, s.counters);
   RICK_CUDA(cudaGetLastError());
-  return scan_bins(s.bin_count, s.item_off, nbins, rule, s.scan_tmp, st);
+  return scan_bins(s.bin_count, s.item_off, nbins, max_chunk, s.scan_tmp, st);
 }
 
 // Lanes that share one row's samples: one for rows of fewer than eight loads (a row
@@ -804,7 +804,7 @@ int bin_rows_batch(const BatchLaunch &b, Scratch &s, uint32_t max_chunk, cudaStr
   k_bin_count_batch<<<blocks_cnt, 256, 0, st>>>(b.jobs, b.njobs, b.u.row_units, units,
                                                 s.bin_count, s.counters);
   RICK_CUDA(cudaGetLastError());
-  RICK_TRY(scan_bins(s.bin_count, s.item_off, nbins, ItemRule{max_chunk, false}, s.scan_tmp, st));
+  RICK_TRY(scan_bins(s.bin_count, s.item_off, nbins, max_chunk, s.scan_tmp, st));
   for (int c = 0; c < b.n_sc; c++) {
     const ScatterClass &k = b.sc[c];
     const int blocks = (int)std::max<uint64_t>(

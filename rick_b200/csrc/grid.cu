@@ -9,7 +9,8 @@
 // records, so that no sum can overflow), and writes the tile once: with
 // plain coalesced stores when the tile is
 // a single item, or with one atomic per non-zero cell when a dense tile was
-// split over several items.  The kernel weights follow w-stacking.cu:162-180:
+// split over several items -- in the mixed form into FP64 sums beside the cube
+// where the items are many (WideTiles).  The kernel weights follow w-stacking.cu:162-180:
 //   u_dist = j + 0.5 - pos_u, table index (int)(5*|u_dist + KernelLen|),
 //   weight tab[jKer]*tab[kKer] (Gaussian / Kaiser-Bessel tables), or
 //   norm*exp(-(u_dist^2+v_dist^2)*std22) (high-precision Gaussian, evaluated
@@ -127,7 +128,8 @@ __device__ __forceinline__ double item_scale(const RecF64 *__restrict__ rec, uin
 // cube and the rows/tile it touched marked.  LPR lanes per record (>= w_support:
 // 8 or 16, or the support itself when it is a compile-time constant that does
 // not divide 32 well -- 9 lanes give three records a warp step where 16 gave
-// two); 32/LPR records per warp step, lanes past RPW*LPR idle.
+// two); 32/LPR records per warp step, lanes past RPW*LPR idle.  wide, wide_done: the
+// tile's FP64 sums and the count of its `items` that are in them (WideTiles; else null).
 template <typename OutT, int LPR, int SUP = 0>
 __device__ __forceinline__ void grid_item(const RecF64 *__restrict__ rec, uint32_t r0, uint32_t r1,
                                           const Geometry &g, bool hi, const double *s_tab,
@@ -136,7 +138,9 @@ __device__ __forceinline__ void grid_item(const RecF64 *__restrict__ rec, uint32
                                           typename Vec2<OutT>::type *__restrict__ cube,
                                           uint32_t *__restrict__ rowmask,
                                           uint32_t *__restrict__ tilemask, FixTile *tile,
-                                          double *s_red, uint32_t *s_rows) {
+                                          double *s_red, uint32_t *s_rows,
+                                          double *wide = nullptr, uint32_t *wide_done = nullptr,
+                                          uint32_t items = 0) {
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const unsigned d = lane % LPR;                 // footprint column / row handled
   const unsigned grp_base = lane - d;            // first lane of this record's group
@@ -217,6 +221,39 @@ __device__ __forceinline__ void grid_item(const RecF64 *__restrict__ rec, uint32
     atomicOr(&tilemask[((uint64_t)w * g.nty + ty) * tmw + (tx >> 5)], 1u << (tx & 31));
   }
   const uint64_t plane = (uint64_t)g.nx * g.ny;
+  if constexpr (sizeof(OutT) == 4) {
+    if (wide) {
+      // The item is added into the tile's FP64 sums; the last one writes the cube (or
+      // adds to it) and leaves the sums at zero.
+      for (int c = threadIdx.x; c < kTile * kTile; c += blockDim.x) {
+        const int cs = (c / kTile) * kPitch + c % kTile;
+        const double vr = fix_value<OutT>(tile->lo_re, tile->hi_re, cs) * inv_scale;
+        const double vi = fix_value<OutT>(tile->lo_im, tile->hi_im, cs) * inv_scale;
+        if (vr != 0.0) atomicAdd(wide + c, vr);
+        if (vi != 0.0) atomicAdd(wide + kTile * kTile + c, vi);
+      }
+      __threadfence();
+      __syncthreads();
+      if (threadIdx.x == 0) *s_rows = atomicAdd(wide_done, 1u);
+      __syncthreads();
+      if (*s_rows != items - 1) return;
+      __threadfence();
+      for (int c = threadIdx.x; c < kTile * kTile; c += blockDim.x) {
+        const int gy = y0 + c / kTile, gx = x0 + c % kTile;
+        const double vr = __ldcg(wide + c), vi = __ldcg(wide + kTile * kTile + c);
+        __stcg(wide + c, 0.0);
+        __stcg(wide + kTile * kTile + c, 0.0);
+        if (gy >= g.ny || gx >= g.nx) continue;
+        const uint64_t idx = (uint64_t)w * plane + (uint64_t)gy * g.nx + gx;
+        float2 o = accumulate ? cube[idx] : make_float2(0.0f, 0.0f);
+        o.x += (float)vr;
+        o.y += (float)vi;
+        cube[idx] = o;
+      }
+      if (threadIdx.x == 0) *wide_done = 0;
+      return;
+    }
+  }
   for (int c = threadIdx.x; c < kTile * kTile; c += blockDim.x) {
     const int y = c / kTile, x = c % kTile;
     const int gy = y0 + y, gx = x0 + x;
@@ -244,6 +281,19 @@ __device__ __forceinline__ void grid_item(const RecF64 *__restrict__ rec, uint32
   }
 }
 
+// Slot of a bin's wide tile: the first of the table, from the bin's hash on, that is
+// free (taken now) or its own; slots: none (wide_slots leaves room for every tile that
+// asks).
+__device__ __forceinline__ uint32_t wide_slot(const WideTiles &t, uint32_t bin) {
+  uint32_t h = (bin * 2654435761u) >> 8;
+  for (uint32_t i = 0; i < t.slots; i++, h++) {
+    h &= t.slots - 1;
+    const uint32_t k = atomicCAS(&t.table[h], 0u, bin + 1);
+    if (k == 0 || k == bin + 1) return h;
+  }
+  return t.slots;
+}
+
 // last bin b with item_off[b] <= item
 __device__ __forceinline__ uint32_t bin_of_item(const uint32_t *__restrict__ item_off,
                                                 uint32_t nbins, uint32_t item) {
@@ -255,21 +305,20 @@ __device__ __forceinline__ uint32_t bin_of_item(const uint32_t *__restrict__ ite
   return lo;
 }
 
-// Items as ItemRule sizes them (the mixed form's parts capped).
 // Six blocks per SM (the launch's grid): registers bounded to 40 a thread
 // (c2 FP64 gridder 1.00 -> 0.955 ms against the compiler's own choice, five).
 template <typename OutT, int LPR, int SUP = 0>
 __global__ void __launch_bounds__(kGridThreads, 6)
     k_grid_tiles(const RecF64 *__restrict__ rec, const uint32_t *__restrict__ bin_off,
-                 const uint32_t *__restrict__ item_off, uint32_t nbins, uint32_t fine,
+                 const uint32_t *__restrict__ item_off, uint32_t nbins, uint32_t max_chunk,
                  Geometry g, int kernel, const double *__restrict__ table, int accumulate,
-                 uint64_t *__restrict__ counters,
+                 uint64_t *__restrict__ counters, WideTiles wt,
                  typename Vec2<OutT>::type *__restrict__ cube, uint32_t *__restrict__ rowmask,
                  uint32_t *__restrict__ tilemask) {
   __shared__ FixTile tile;
   __shared__ double s_tab[kIncreasePrecision * kMaxSupport];
   __shared__ double s_red[kGridThreads / 32];
-  __shared__ uint32_t s_item, s_bin, s_first, s_nitems, s_rows;
+  __shared__ uint32_t s_item, s_bin, s_first, s_nitems, s_rows, s_slot;
 
   const int ntab = kIncreasePrecision * g.support;
   for (int t = threadIdx.x; t < ntab; t += blockDim.x) s_tab[t] = table[t];
@@ -286,6 +335,8 @@ __global__ void __launch_bounds__(kGridThreads, 6)
         bin = bin_of_item(item_off, nbins, item);
         s_first = item_off[bin];
         s_nitems = item_off[bin + 1] - item_off[bin];
+        if (sizeof(OutT) == 4)
+          s_slot = s_nitems > kWideParts ? wide_slot(wt, bin) : wt.slots;
       }
       s_item = item;
       s_bin = bin;
@@ -300,11 +351,13 @@ __global__ void __launch_bounds__(kGridThreads, 6)
     const int tx = (int)(bin % (uint32_t)g.ntx);
     const int ty = (int)((bin / (uint32_t)g.ntx) % (uint32_t)g.nty);
     const int w = (int)(bin / ((uint32_t)g.ntx * (uint32_t)g.nty));
-    const uint32_t c0 = bin_off[bin], c1 = bin_off[bin + 1];
-    const uint32_t per = ItemRule::size<sizeof(OutT) == 4>(fine, c1 - c0);
-    const uint32_t r0 = c0 + chunk * per, r1 = min(c1, r0 + per);
+    const uint32_t r0 = bin_off[bin] + chunk * max_chunk;
+    const uint32_t r1 = min(bin_off[bin + 1], r0 + max_chunk);
+    const bool wide = sizeof(OutT) == 4 && s_slot < wt.slots;
     grid_item<OutT, LPR, SUP>(rec, r0, r1, g, hi, s_tab, ntab, wmax, tx, ty, w, s_nitems == 1,
-                         accumulate, cube, rowmask, tilemask, &tile, s_red, &s_rows);
+                         accumulate, cube, rowmask, tilemask, &tile, s_red, &s_rows,
+                         wide ? wt.sums + (uint64_t)s_slot * (2 * kTile * kTile) : nullptr,
+                         wt.done + (wide ? s_slot : 0), s_nitems);
     __syncthreads();
   }
 }
@@ -436,7 +489,7 @@ __global__ void k_zero_split_tiles_batch(const BatchJob *__restrict__ jobs, int 
 
 template <typename OutT>
 int launch_grid(const Geometry &g, int kernel, Scratch &s, void *cube, int accumulate,
-                ItemRule rule, cudaStream_t st, uint32_t *rowmask, uint32_t *tilemask) {
+                uint32_t max_chunk, cudaStream_t st, uint32_t *rowmask, uint32_t *tilemask) {
   const int sms = num_sms();
   using V = typename Vec2<OutT>::type;
   const uint32_t nbins = (uint32_t)g.nbins();
@@ -445,8 +498,8 @@ int launch_grid(const Geometry &g, int kernel, Scratch &s, void *cube, int accum
   RICK_LAUNCHED();
 #define RICK_GRID(LPR, SUP)                                                                    \
   k_grid_tiles<OutT, LPR, SUP><<<blocks, kGridThreads, 0, st>>>(                               \
-      s.records, s.bin_count, s.item_off, nbins, rule.fine, g, kernel, s.table, accumulate,         \
-      s.counters, (V *)cube, rowmask, tilemask)
+      s.records, s.bin_count, s.item_off, nbins, max_chunk, g, kernel, s.table, accumulate,    \
+      s.counters, s.wide, (V *)cube, rowmask, tilemask)
   // the common supports unrolled (7: 1.16 -> 1.00 ms FP64 at 4096^2 x 32; 9
   // with 9 lanes a record: 1.73 -> 1.20 ms at 8192^2 x 64)
   if (g.support == 7)
@@ -465,11 +518,11 @@ int launch_grid(const Geometry &g, int kernel, Scratch &s, void *cube, int accum
 }  // namespace
 
 int grid_tiles(const Geometry &g, int kernel, int precision, Scratch &s, void *cube,
-               int accumulate, ItemRule rule, cudaStream_t st, uint32_t *rowmask,
+               int accumulate, uint32_t max_chunk, cudaStream_t st, uint32_t *rowmask,
                uint32_t *tilemask) {
   if (precision == RICK_PREC_FP64)
-    return launch_grid<double>(g, kernel, s, cube, accumulate, rule, st, rowmask, tilemask);
-  return launch_grid<float>(g, kernel, s, cube, accumulate, rule, st, rowmask, tilemask);
+    return launch_grid<double>(g, kernel, s, cube, accumulate, max_chunk, st, rowmask, tilemask);
+  return launch_grid<float>(g, kernel, s, cube, accumulate, max_chunk, st, rowmask, tilemask);
 }
 
 int zero_split_tiles(const Geometry &g, int precision, Scratch &s, void *cube, cudaStream_t st) {

@@ -190,12 +190,12 @@ int rick_wstack_noalloc(int num_w_planes, uint64_t num_points, uint32_t freq_per
   RICK_CUDA(cudaMemsetAsync(s.bin_count, 0, (nbins + 1) * sizeof(uint32_t), st));
   RICK_CUDA(cudaMemsetAsync(s.bin_cursor, 0, nbins * sizeof(uint32_t), st));
   const uint64_t per = num_points / ((uint64_t)num_sms() * 4 + 1);
-  const ItemRule rule{(uint32_t)(per < 1024 ? 1024 : (per > 8192 ? 8192 : per)), false};
-  RICK_TRY(bin_count_rows(g, num_points, uu, vv, ww, s, rule, st));
+  const uint32_t chunk = (uint32_t)(per < 1024 ? 1024 : (per > 8192 ? 8192 : per));
+  RICK_TRY(bin_count_rows(g, num_points, uu, vv, ww, s, chunk, st));
   RICK_TRY(bin_scatter_rows(g, num_points, uu, vv, ww, weight, vis_real, vis_img, freq_per_chan,
                             polarizations, s, st));
   RICK_CUDA(cudaMemsetAsync(grid, 0, 2ull * num_w_planes * grid_size_x * grid_size_y * 8, st));
-  RICK_TRY(grid_tiles(g, kernel, RICK_PREC_FP64, s, grid, 0, rule, st));
+  RICK_TRY(grid_tiles(g, kernel, RICK_PREC_FP64, s, grid, 0, chunk, st));
   return RICK_OK;
 }
 

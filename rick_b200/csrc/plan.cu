@@ -139,7 +139,7 @@ struct rick_plan {
   double *d_img = nullptr;     // [2*Ny*Nx] image staging for host calls
   double *d_stage = nullptr;   // conversion staging for mixed import/export
   void *d_norm = nullptr;      // NORMALIZE_UVW scratch (extrema)
-  ItemRule items{1024, false};  // gridder work items of the current gridding
+  uint32_t chunk = 1024;       // gridder records per work item of the current gridding
   // streaming ingest (rick_plan_ingest_*): rows staged in h_rows_d, samples by slices
   bool ingest = false;
   uint64_t ing_rows = 0, ing_next = 0;
@@ -259,18 +259,31 @@ int choose_fft(rick_plan *p) {
   return RICK_OK;
 }
 
-// Records per gridder work item: rows / (8 per SM), within 64..1024 (more for dense
-// tiles in the mixed form, ItemRule).  A job's dense
+// Records per gridder work item: rows / (8 per SM), within 64..1024.  A job's dense
 // tiles are split finely enough to occupy every block slot of the gridder (six an
 // SM) when rows are few -- items of 1024 left 31 of 888 slots with work at 5,418
 // rows (47 -> 14 us) and 979 for 888 at 279,800 (86 -> 65 us) -- while above 1024
 // the last items' tail grows (5.1M rows, 4096^2 x 32: 0.96 ms at 8192, 0.87 at
 // 4096, 0.80 at 1024) and below it the per-item cost does (0.81 ms at 512, 0.88 at
 // 256).
-ItemRule choose_items(uint64_t nrows, int precision) {
+uint32_t choose_chunk(uint64_t nrows) {
   const uint64_t per = nrows / ((uint64_t)num_sms() * 8);
-  return {(uint32_t)std::min<uint64_t>(1024, std::max<uint64_t>(64, per)),
-          precision == RICK_PREC_MIXED};
+  return (uint32_t)std::min<uint64_t>(1024, std::max<uint64_t>(64, per));
+}
+
+// Slots for the wide tiles of a mixed plan: tiles of more than kWideParts items of
+// choose_chunk(rows) records, of at most four records a row.  Items of 64 records make
+// that at most rows / 1024; longer ones below 1024 (a whole number, at most rows / (8 per
+// SM)) at most half a tile an SM and 1/64 more; and items of 1024 rows / 16,384.
+uint32_t wide_slots(uint64_t max_rows, uint64_t nbins) {
+  const uint64_t records = 4 * max_rows;
+  const uint64_t most =
+      std::min({nbins, records / (kWideParts * 64),
+                std::max<uint64_t>((uint64_t)num_sms(), records / (kWideParts * 1024) + 1)});
+  if (most == 0) return 0;
+  uint32_t slots = 1;
+  while (slots < most + most / 4) slots *= 2;
+  return slots;
 }
 
 int ensure_lm(rick_plan *p, int xaxis, int yaxis, int xtot, int ytot, double resolution,
@@ -345,8 +358,8 @@ int grid_begin(rick_plan *p, uint64_t nrows, const double *uu, const double *vv,
     RICK_TRY(normalize_uvw(nrows, const_cast<double *>(uu), const_cast<double *>(vv),
                            const_cast<double *>(ww), p->d_norm, st));
   RICK_CUDA(cudaMemsetAsync(p->d_clear, 0, p->clear_bytes, st));
-  p->items = choose_items(nrows, p->d.precision);
-  RICK_TRY(bin_count_rows(p->g, nrows, uu, vv, ww, p->s, p->items, st));
+  p->chunk = choose_chunk(nrows);
+  RICK_TRY(bin_count_rows(p->g, nrows, uu, vv, ww, p->s, p->chunk, st));
   return mark(p, p->ev[1], st);
 }
 
@@ -366,7 +379,7 @@ int grid_finish(rick_plan *p, uint64_t nrows, int accumulate, bool sparse, cudaS
     RICK_CUDA(cudaMemsetAsync(p->cube, 0, p->cube_vals * p->val_bytes, st));
   }
   RICK_TRY(mark(p, p->ev[3], st));
-  RICK_TRY(grid_tiles(p->g, p->d.kernel, p->d.precision, p->s, p->cube, accumulate, p->items,
+  RICK_TRY(grid_tiles(p->g, p->d.kernel, p->d.precision, p->s, p->cube, accumulate, p->chunk,
                       st, sparse ? p->f.rowmask : nullptr, sparse ? p->f.tilemask : nullptr));
   RICK_TRY(mark(p, p->ev[4], st));
   p->ran[0] = p->ran[1] = p->ran[3] = true;
@@ -487,6 +500,8 @@ int rick_plan_footprint(const rick_plan_desc *desc, uint64_t *bytes) {
     b += std::max<uint64_t>(b / 4, 512ull << 20);          // cuFFT work (upper bound)
   b += 4 * (nbins + 1) * 4 + 4 * scan_tmp_words(nbins + 1);  // bins, items, cursor, scan
   b += 4 * desc->max_rows * sizeof(RecF64);                // records
+  if (desc->precision == RICK_PREC_MIXED)
+    b += (uint64_t)wide_slots(desc->max_rows, nbins) * (2 * kTile * kTile * sizeof(double) + 8);
   b += (nx + ny) * 8 + 64;
   *bytes = b;
   return RICK_OK;
@@ -520,7 +535,20 @@ int rick_plan_create(rick_plan **out, const rick_plan_desc *desc) {
   A((void **)&p->s.item_off, (nbins + 1) * 4);
   A((void **)&p->s.scan_tmp, scan_tmp_words(nbins + 1) * 4);
   p->s.max_records = 4 * std::max<uint64_t>(desc->max_rows, 1);
-  A((void **)&p->s.records, p->s.max_records * sizeof(RecF64));
+  // the records and, mixed, the wide tiles' sums behind them
+  WideTiles &wide = p->s.wide;
+  if (desc->precision == RICK_PREC_MIXED) wide.slots = wide_slots(desc->max_rows, nbins);
+  const size_t rec_bytes = p->s.max_records * sizeof(RecF64);
+  const size_t sum_bytes = (size_t)wide.slots * 2 * kTile * kTile * sizeof(double);
+  const size_t wide_bytes = sum_bytes + wide.slots * sizeof(uint32_t);
+  A((void **)&p->s.records, rec_bytes + wide_bytes);
+  if (st == RICK_OK && wide.slots) {
+    wide.sums = (double *)((char *)p->s.records + rec_bytes);
+    wide.done = (uint32_t *)((char *)wide.sums + sum_bytes);
+    // (done before the copies from pageable memory below return)
+    const cudaError_t e = cudaMemset(wide.sums, 0, wide_bytes);
+    if (e != cudaSuccess) st = cuda_status(e, "cudaMemset(wide tiles)", __FILE__, __LINE__);
+  }
   A((void **)&p->s.table, kIncreasePrecision * kMaxSupport * 8);
   A((void **)&p->d_lm, (size_t)(desc->grid_size_x + desc->grid_size_y) * 8);
   if (st == RICK_OK) {
@@ -544,6 +572,7 @@ int rick_plan_create(rick_plan **out, const rick_plan_desc *desc) {
     } part[] = {{(void **)&p->s.counters, kNumCounters * 8},
                 {(void **)&p->s.bin_count, (nbins + 1) * 4},
                 {(void **)&p->s.bin_cursor, nbins * 4},
+                {(void **)&p->s.wide.table, p->s.wide.slots * 4},
                 {(void **)&p->f.rowmask, p->sparse ? masks * 4 : 0},
                 {(void **)&p->f.tilemask, p->sparse ? tiles * 4 : 0},
                 {(void **)&p->f.counts, p->sparse ? (size_t)(1 + nwl) * 4 : 0}};

@@ -84,6 +84,24 @@ struct __align__(32) RecF64 {
   double pu, pv;     // pixel position
 };
 
+// FP64 sums of a mixed plan's densest tiles: of those with more than kWideParts work
+// items (grid.cu).  An FP32 cell loses about sqrt(items / 3) of an add's rounding to the
+// items added into it, and larger items lose more in their own 32-bit sums.  Error of
+// images against 64 bits, 64^2 on one plane, three array layouts, sources and noise:
+// 75,000 rows 1.3, 1.3 and 1.3e-7 (added into FP32 cells 3.1, 3.2 and 4.1e-7 with items
+// of 64 records, 3.1, 2.5 and 2.1e-7 with 1024); noise alone 1.7, 1.8 and 1.8e-7 (4.1,
+// 3.8 and 4.5e-7 with 64, 18, 17 and 19e-7 with 1024).  The adds of that many items at
+// one tile's addresses take longer in FP64 (93 -> 103 us a call; real and imaginary sums
+// apart, since interleaved they touch twice the sectors: 126); 300,000 rows on 128^2 x 2
+// 145 -> 141.  A tile takes the slot of a hash table that its bin finds first.
+constexpr uint32_t kWideParts = 64;
+struct WideTiles {
+  uint32_t *table = nullptr;  // [slots] bin + 1, or 0: cleared before every gridding
+  uint32_t *done = nullptr;   // [slots] items added; 0 between griddings
+  double *sums = nullptr;     // [slots][re, im][kTile^2]; 0 between griddings
+  uint32_t slots = 0;         // a power of two
+};
+
 // Device scratch owned by a plan.
 struct Scratch {
   uint32_t *bin_count = nullptr;   // [nbins+1] counts, then exclusive offsets
@@ -94,36 +112,7 @@ struct Scratch {
   RecF64 *records = nullptr;       // [max_records]
   uint64_t max_records = 0;
   double *table = nullptr;         // 1-D kernel table, 5*support doubles
-};
-
-// Records per gridder work item of a tile with c records: `fine`, but in the mixed
-// form (cap_parts) so many that a tile of more than kParts items has at most kParts of
-// up to 1024 records, or 2 kParts of up to 4096, powers of two so that the scan of all
-// bins divides by `fine` alone.  Every item is added into FP32 cells, which lose about
-// sqrt(items / 3) of an add's rounding on the way, while the items' own 32-bit sums
-// lose the more the more records they hold (grid.cu).  Error of images against 64
-// bits, 64^2 on one plane, three array layouts: 75,000 rows 2.1, 2.0 and 2.0e-7 (3.1,
-// 3.2 and 4.1e-7 with items of 64 throughout, 3.1, 2.5 and 2.1e-7 with 1024); 5M rows
-// 4.5, 3.8 and 4.1e-7 (6.4, 6.0 and 8.4e-7 with 1024, 8.0, 5.2 and 5.8e-7 with 8192).
-// Half as many parts cost time where a tile holds much of a job (100,000 rows, 1024^2,
-// one plane, support 15: 234 us a call against 178, and 161 uncapped).  FP64 cells and
-// sums lose nothing that shows.
-struct ItemRule {
-  static constexpr uint32_t kParts = 128;
-  uint32_t fine;  // at most 1024 with cap_parts
-  bool cap_parts;
-  // log2 of the size of a capped tile's items: c / 128 up to 1024, or c / 256 up to 4096
-  // where that is more, rounded up to powers of two
-  static __device__ __forceinline__ uint32_t size_log(uint32_t c) {
-    const uint32_t part = 32 - __clz((c - 1) / kParts), few = 32 - __clz((c - 1) / (2 * kParts));
-    return max(min(part, 10u), min(few, 12u));
-  }
-  template <bool CAP> static __device__ __forceinline__ bool capped(uint32_t fine, uint32_t c) {
-    return CAP && c > kParts * fine;  // c > 8192
-  }
-  template <bool CAP> static __device__ __forceinline__ uint32_t size(uint32_t fine, uint32_t c) {
-    return capped<CAP>(fine, c) ? 1u << size_log(c) : fine;
-  }
+  WideTiles wide;                  // of a plan in the mixed form
 };
 
 // Scratch of the sparse-aware FFT (fft.cu).
@@ -223,14 +212,14 @@ void make_table(int kernel, int support, double *tab);
 // Pipeline stages (bin.cu, grid.cu, phase.cu).
 // Both passes expect bin_count [nbins + 1] and bin_cursor [nbins] cleared.
 int bin_count_rows(const Geometry &g, uint64_t nrows, const double *uu, const double *vv,
-                   const double *ww, Scratch &s, ItemRule rule, cudaStream_t st);
+                   const double *ww, Scratch &s, uint32_t max_chunk, cudaStream_t st);
 // The samples of all counted rows, or of successive slices of them.
 int bin_scatter_rows(const Geometry &g, uint64_t nrows, const double *uu, const double *vv,
                      const double *ww, const float *weight, const float *vis_re,
                      const float *vis_im, uint32_t nchan, uint32_t npol, Scratch &s,
                      cudaStream_t st);
 int grid_tiles(const Geometry &g, int kernel, int precision, Scratch &s, void *cube,
-               int accumulate, ItemRule rule, cudaStream_t st,
+               int accumulate, uint32_t max_chunk, cudaStream_t st,
                uint32_t *rowmask = nullptr, uint32_t *tilemask = nullptr);
 // Zeroes the tiles that several work items add into (the sparse path does not
 // clear the cube).
@@ -251,8 +240,8 @@ int phase_sum(int precision, const void *cube, int xaxis, int yaxis, int nw, int
 int normalize_uvw(uint64_t n, double *uu, double *vv, double *ww, void *scratch,
                   cudaStream_t st);
 // counts[0..nbins) -> exclusive offsets in place (counts[nbins] the total) and
-// item_off[0..nbins]: exclusive offsets of the bins' work items (scan.cu).
-int scan_bins(uint32_t *counts, uint32_t *item_off, uint64_t nbins, ItemRule rule,
+// item_off[0..nbins]: exclusive offsets of ceil(count / max_chunk) (scan.cu).
+int scan_bins(uint32_t *counts, uint32_t *item_off, uint64_t nbins, uint32_t max_chunk,
               uint32_t *tmp, cudaStream_t st);
 uint64_t scan_tmp_words(uint64_t n);
 

@@ -1,5 +1,5 @@
 // Offsets of the bins and of the gridder's work items: exclusive prefix sums of the
-// record counts and of the bins' items (ItemRule), both at once.  One block for up to
+// record counts and of ceil(count / max_chunk), both at once.  One block for up to
 // 8191 bins; beyond, a first kernel sums blocks of 8192 bins and a second adds the
 // sums before its block (read by every block: 512 at 4M bins) to the
 // block's own scan.  The scans of one sum at a time this replaces took seven
@@ -48,51 +48,28 @@ __device__ __forceinline__ Sum2 block_exclusive(Sum2 v, Sum2 &total) {
   return warp == 0 ? own : own + before;
 }
 
-// Items of a thread's bins, v[k].rec records each.  The rare capped tile is left to
-// code off the path (in line it added 2 us to the scans: they run from a cold
-// instruction cache).
-template <bool CAP>
-__device__ __forceinline__ Sum2 count_items(Sum2 (&v)[kScanPerThread], uint32_t fine) {
-  uint32_t most = 0;
-  Sum2 sum = {0, 0};
-#pragma unroll
-  for (int k = 0; k < kScanPerThread; k++) {
-    v[k].items = (v[k].rec + fine - 1) / fine;
-    most = max(most, v[k].rec);
-    sum = sum + v[k];
-  }
-  if (__builtin_expect(ItemRule::capped<CAP>(fine, most), false)) {
-    sum.items = 0;
-#pragma unroll
-    for (int k = 0; k < kScanPerThread; k++) {
-      const uint32_t c = v[k].rec, log = ItemRule::size_log(max(c, 4 * ItemRule::kParts));
-      if (ItemRule::capped<CAP>(fine, c)) v[k].items = (c + (1u << log) - 1) >> log;
-      sum.items += v[k].items;
-    }
-  }
-  return sum;
+__device__ __forceinline__ Sum2 bin_sum(uint32_t c, uint32_t max_chunk) {
+  return {c, (c + max_chunk - 1) / max_chunk};
 }
 
-template <bool CAP>
 __global__ void __launch_bounds__(kScanThreads)
-    k_scan_sums(const uint32_t *__restrict__ counts, uint64_t nbins, uint32_t fine,
+    k_scan_sums(const uint32_t *__restrict__ counts, uint64_t nbins, uint32_t max_chunk,
                 Sum2 *__restrict__ sums) {
   const uint64_t base = (uint64_t)blockIdx.x * kScanBlock + threadIdx.x;
-  Sum2 v[kScanPerThread], total;
+  Sum2 local = {0, 0}, total;
 #pragma unroll
   for (int k = 0; k < kScanPerThread; k++) {
     const uint64_t i = base + (uint64_t)k * kScanThreads;
-    v[k].rec = i < nbins ? counts[i] : 0u;
+    if (i < nbins) local = local + bin_sum(counts[i], max_chunk);
   }
-  block_exclusive(count_items<CAP>(v, fine), total);
+  block_exclusive(local, total);
   if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
 // sums: the totals of the blocks (null for a single block).
-template <bool CAP>
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_bins(uint32_t *__restrict__ counts, uint32_t *__restrict__ item_off, uint64_t nbins,
-                uint32_t fine, const Sum2 *__restrict__ sums) {
+                uint32_t max_chunk, const Sum2 *__restrict__ sums) {
   Sum2 before = {0, 0}, total;
   if (sums) {
     Sum2 part = {0, 0};
@@ -100,10 +77,13 @@ __global__ void __launch_bounds__(kScanThreads)
     block_exclusive(part, before);
   }
   const uint64_t base = (uint64_t)blockIdx.x * kScanBlock + (uint64_t)threadIdx.x * kScanPerThread;
-  Sum2 v[kScanPerThread];
+  Sum2 v[kScanPerThread], local = {0, 0};
 #pragma unroll
-  for (int k = 0; k < kScanPerThread; k++) v[k].rec = base + k < nbins ? counts[base + k] : 0u;
-  Sum2 run = before + block_exclusive(count_items<CAP>(v, fine), total);
+  for (int k = 0; k < kScanPerThread; k++) {
+    v[k] = bin_sum(base + k < nbins ? counts[base + k] : 0u, max_chunk);
+    local = local + v[k];
+  }
+  Sum2 run = before + block_exclusive(local, total);
 #pragma unroll
   for (int k = 0; k < kScanPerThread; k++) {
     if (base + k <= nbins) {  // entry nbins: the totals
@@ -126,28 +106,19 @@ uint64_t scan_tmp_words(uint64_t n) {
   return words + 64;
 }
 
-namespace {
-template <bool CAP>
-int launch_scan(uint32_t *counts, uint32_t *item_off, uint64_t nbins, uint32_t fine, uint32_t *tmp,
-                cudaStream_t st) {
+int scan_bins(uint32_t *counts, uint32_t *item_off, uint64_t nbins, uint32_t max_chunk,
+              uint32_t *tmp, cudaStream_t st) {
   const uint64_t nb = (nbins + 1 + kScanBlock - 1) / kScanBlock;
   Sum2 *sums = nb > 1 ? (Sum2 *)tmp : nullptr;
   if (sums) {
     RICK_LAUNCHED();
-    k_scan_sums<CAP><<<(unsigned)nb, kScanThreads, 0, st>>>(counts, nbins, fine, sums);
+    k_scan_sums<<<(unsigned)nb, kScanThreads, 0, st>>>(counts, nbins, max_chunk, sums);
     RICK_CUDA(cudaGetLastError());
   }
   RICK_LAUNCHED();
-  k_scan_bins<CAP><<<(unsigned)nb, kScanThreads, 0, st>>>(counts, item_off, nbins, fine, sums);
+  k_scan_bins<<<(unsigned)nb, kScanThreads, 0, st>>>(counts, item_off, nbins, max_chunk, sums);
   RICK_CUDA(cudaGetLastError());
   return RICK_OK;
-}
-}  // namespace
-
-int scan_bins(uint32_t *counts, uint32_t *item_off, uint64_t nbins, ItemRule rule, uint32_t *tmp,
-              cudaStream_t st) {
-  return rule.cap_parts ? launch_scan<true>(counts, item_off, nbins, rule.fine, tmp, st)
-                        : launch_scan<false>(counts, item_off, nbins, rule.fine, tmp, st);
 }
 
 }  // namespace rick
