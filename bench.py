@@ -57,17 +57,26 @@ WORKLOAD_TEXT = {
 # captures of a kernel on a workload at full size, keyed by (workload, kernel);
 # each entry names the capture.  A kernel without a capture reports null.
 NCU_TRAFFIC = {
-    ("c2", "k_bin_scatter<32,1>"): (10_851_913_216, "profiles/traffic_c2.md"),
+    ("c2", "k_bin_scatter<32,4,0>"): (10_853_461_632, "profiles/traffic_c2.md"),
+    ("c2", "k_fft_cols<double,12> + k_fft_finish<double,12>"): (2_859_332_992,
+                                                               "profiles/traffic_c2.md"),
 }
 
 
-def plan_kernel_name(stage, nx, ny):
-    """The kernel behind a plan stage on the sparse-aware path (FP64)."""
+def plan_kernel_name(stage, nx, ny, nv, npol, support):
+    """The kernels behind a whole-cube plan's stage on the sparse-aware path (FP64) for
+    rows of nv samples at 16-byte boundaries."""
     ly = max(int(ny).bit_length() - 1, 0)
     lx = max(int(nx).bit_length() - 1, 0)
-    return {"bin_count": "k_bin_count", "bin_scatter": "k_bin_scatter<32,1>",
-            "cube_zero": "k_zero_split_tiles<double>", "grid": "k_grid_tiles<double,8>",
-            "fft": f"k_fft_rows<double,{lx}>", "phase": f"k_fft_cols<double,{ly}>"}.get(stage, stage)
+    vec = 4 if nv % 4 == 0 and npol in (1, 2, 4) else 2 if nv % 2 == 0 and npol in (1, 2) else 1
+    loads = nv // vec
+    lanes = 1 if loads < 8 else 4 if loads < 16 else 16 if loads < 32 else 32
+    scatter = (f"k_bin_scatter<{lanes},{vec},0>" if lanes > 1 else f"k_bin_scatter_short<{vec}>")
+    grid = {7: "8,7", 9: "9,9"}.get(support, "8,0" if support <= 8 else "16,0")
+    phase = f"k_fft_cols<double,{ly}>" + (f" + k_fft_finish<double,{ly}>" if ly >= 10 else "")
+    return {"bin_count": "k_bin_count", "bin_scatter": scatter,
+            "cube_zero": "k_zero_split_tiles<double>", "grid": f"k_grid_tiles<double,{grid}>",
+            "fft": f"k_fft_rows<double,{lx}>", "phase": phase}.get(stage, stage)
 
 
 def fp64_gemm_tflops(dev) -> float:
@@ -375,7 +384,7 @@ def run_ours(args):
                             stats64.get("fft_rows", 0))
     dom = max(stage64, key=stage64.get)
     achieved = alg[dom] / (stage64[dom] * 1e-3) / 1e9
-    kname = plan_kernel_name(dom, nx, ny)
+    kname = plan_kernel_name(dom, nx, ny, nv, npol, cfg.w_support)
     traffic = NCU_TRAFFIC.get((args.workload, kname)) if not args.time_fraction < 1 else None
     roofline = {"kernel": dom, "kernel_name": kname,
                 "bound": "hbm", "achieved": round(achieved, 1),

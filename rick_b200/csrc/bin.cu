@@ -337,7 +337,7 @@ __device__ __forceinline__ void row_sums(const float *__restrict__ wrow,
 // one row's samples in loads of N; after G rounds every lane holds the sum of "its"
 // row, and the records are scattered one row per lane with warp-combined cursor
 // increments.  HBM-bound for long rows (5.1M rows of 256 samples: 10.8 GB in 1.75 ms,
-// 0.95 of the measured copy rate); rows of eight loads run four lanes a row (3.8M
+// 0.96 of the measured copy rate); rows of eight loads run four lanes a row (3.8M
 // rows of 32 samples: 0.29 ms, against 0.72 with a lane a row and 0.35 with eight).
 template <int G, int N, bool SHARD>
 __device__ __forceinline__ void scatter_rows(

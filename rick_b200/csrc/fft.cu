@@ -432,9 +432,9 @@ __global__ void __launch_bounds__(Shape<L>::kThreads, row_min_blocks<L>())
 // which is what TMEM holds, too.  Bounds per plane and 4096-point unit: FP64 (or
 // packed FP32) issue 2,600 cycles of a sub-partition, load/store pipe ~3,600 of
 // the SM (two exchanges 2,048, a wavefront per touched row ~1,130, the image);
-// with 16 warps an SM the two overlap in part: 5,850 measured.  Against two
-// columns a block in radix-8 passes: 3.42 -> 2.60 ms FP64 and 2.55 -> 1.31 mixed
-// (4096^2 x 32), 10.5 -> 6.9 ms FP64 (8192^2, 16 planes of 64) and 10.9 -> 6.3
+// with 16 warps an SM the two overlap in part: 5,300 measured.  With the finish, against
+// two columns a block in radix-8 passes: 3.42 -> 2.49 ms FP64 and 2.55 -> 1.29 mixed
+// (4096^2 x 32), 10.5 -> 6.6 ms FP64 (8192^2, 16 planes of 64) and 10.9 -> 6.3
 // mixed (8192^2 x 32).  Warp w of a block reaches lanes 32 (w % 4) ..
 // +31 (its lane quarter); the warps of one quarter split its columns.
 
